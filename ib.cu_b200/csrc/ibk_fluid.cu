@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include "ibk_internal.h"
 
@@ -67,36 +68,35 @@ __device__ __forceinline__ void face_coords(long long idx, int P0, int P1, int& 
 	}
 }
 
-// op 0: L u, 1: I~ u, 2: H u with H = I~ - lambda L, 3: wa r - H u, 4: wa r -
-// H (wb r) with u = r (the steps of the Chebyshev preconditioner, whose
-// first step's wb r is formed per loaded value instead of stored), per face
+// op 0: L u, 1: I~ u, 2: H u with H = I~ - lambda L, 3: the right-hand side
+// of the solve, k I~ f + kmu (L u + rhs0) (diffusion.h:51-53: gemv(1, L, u,
+// 1, rhs), then gemv(k, I~, f, k mu, rhs)), per face
 //     (L u) = Iz Iy (Lx u) + Iz (Ly u) Ix + (Lz u) Iy Ix
 // with (L_d u) = lo u[-1] + diag u + hi u[+1] along axis d (wrapping on a
-// periodic axis).  Each thread marches along z through kMarchZ planes of one
+// periodic axis).  Each thread marches along z through zrun planes of one
 // (x, y) column: its x and y coefficients and neighbour offsets are taken
 // once, the z neighbours move through registers (one new load per face), and
 // no face needs a division for its coordinates.  A block is 32 columns along
 // x (one warp, coalesced) by 8 along y.  With dot != nullptr the per-block
-// partial sums of u . out (ops 0-2) or r . out (ops 3, 4) go to dot[block]
-// (fixed order).
+// partial sums of u . out go to dot[block] (fixed order).  zrun is 16 where
+// that gives four blocks per SM, else shorter (march_run): a 64^3 grid has
+// only 64 blocks of 16 planes.
 constexpr int kMarchX = 32, kMarchY = 8, kMarchZ = 16;
 
 template <int OP, int DIMS>
 __global__ void __launch_bounds__(kMarchX * kMarchY, 5)
 march_apply_kernel(FluidOps o, const double* __restrict__ u, double* __restrict__ out, double* __restrict__ dot,
-                   const double* __restrict__ rr, double wa, double wb)
+                   int zrun, const double* __restrict__ f, const double* __restrict__ rhs0, double kf, double kmu)
 {
 	constexpr int op = OP;
-	// a loaded value of the operand: wb r for op 4, else u itself
-	auto ld = [wb](const double* p) { return OP == 4 ? wb * *p : *p; };
 	__shared__ double red[kMarchY];
 	const int P0 = o.ax[0].P;
 	const int P1 = DIMS > 1 ? o.ax[1].P : 1;
 	const int P2 = DIMS > 2 ? o.ax[2].P : 1;
 	const int i = blockIdx.x * kMarchX + threadIdx.x;
 	const int j = blockIdx.y * kMarchY + threadIdx.y;
-	const int k0 = blockIdx.z * kMarchZ;
-	const int k1 = min(k0 + kMarchZ, P2);
+	const int k0 = blockIdx.z * zrun;
+	const int k1 = min(k0 + zrun, P2);
 	double acc = 0.0;
 	if (i < P0 && j < P1) {
 		// 32-bit offsets: the plan's grids hold fewer than 2^31 faces
@@ -121,44 +121,43 @@ march_apply_kernel(FluidOps o, const double* __restrict__ u, double* __restrict_
 		const bool zper = o.ax[2].periodic;
 		const int base = i + j * sy + k0 * sz;
 		const double* __restrict__ pu = u + base;      // this column at plane k
-		const double* __restrict__ pr = OP == 3 ? rr + base : nullptr;   // op 4: r is u itself
+		const double* __restrict__ pf = OP == 3 ? f + base : nullptr;
+		const double* __restrict__ pr = OP == 3 ? rhs0 + base : nullptr;
 		double* __restrict__ po = out + base;
 		// register window along z: uzm, uc, uzp = planes k - 1, k, k + 1 (wrapped
 		// on a periodic axis, 0 past a wall), and the plane after next loaded
 		// one iteration ahead
-		double uc = ld(pu);
+		double uc = *pu;
 		double uzm = 0.0, uzp = 0.0;
 		if (DIMS > 2) {
-			uzm = k0 > 0 ? ld(pu - sz) : (zper ? ld(pu + (P2 - 1) * sz) : 0.0);
-			uzp = k0 + 1 < P2 ? ld(pu + sz) : (zper ? ld(pu + (1 - P2) * sz) : 0.0);
+			uzm = k0 > 0 ? pu[-sz] : (zper ? pu[(P2 - 1) * sz] : 0.0);
+			uzp = k0 + 1 < P2 ? pu[sz] : (zper ? pu[(1 - P2) * sz] : 0.0);
 		}
 		for (int k = k0; k < k1; ++k) {
 			double unx = 0.0;
 			if (DIMS > 2 && k + 1 < k1)      // k + 2 <= P2: plane k + 2, or plane 0 past a periodic end
-				unx = k + 2 < P2 ? ld(pu + 2 * sz) : (zper ? ld(pu + (2 - P2) * sz) : 0.0);
+				unx = k + 2 < P2 ? pu[2 * sz] : (zper ? pu[(2 - P2) * sz] : 0.0);
 			const double iz = DIMS > 2 ? zc[3 * P2 + k] : 1.0;
 			double v = 0.0;
 			if (op != 1) {
-				const double um = has_xm ? ld(pu + dxm) : 0.0, up = has_xp ? ld(pu + dxp) : 0.0;
+				const double um = has_xm ? pu[dxm] : 0.0, up = has_xp ? pu[dxp] : 0.0;
 				double l = iz * iy * (xl * um + xd * uc + xh * up);
 				if (DIMS > 1) {
-					const double vm = has_ym ? ld(pu + dym) : 0.0, vp = has_yp ? ld(pu + dyp) : 0.0;
+					const double vm = has_ym ? pu[dym] : 0.0, vp = has_yp ? pu[dyp] : 0.0;
 					l += iz * (yl * vm + yd * uc + yh * vp) * ix;
 				}
 				if (DIMS > 2) l += (zc[k] * uzm + zc[P2 + k] * uc + zc[2 * P2 + k] * uzp) * iy * ix;
 				v = l;
 			}
 			if (op == 1) v = iz * iy * ix * uc;
-			if (op >= 2) v = iz * iy * ix * uc - o.lambda * v;
-			if constexpr (OP >= 3) {
-				// gemv(-1, H, s, w, t) with t = r: -(H s) + w r
-				const double rc = OP == 3 ? *pr : *pu;
-				v = wa * rc - v;
-				if (dot) acc += rc * v;
-				if (OP == 3) pr += sz;
-			} else {
-				if (dot) acc += uc * v;
+			if (op == 2) v = iz * iy * ix * uc - o.lambda * v;
+			if constexpr (OP == 3) {
+				const double idf = iz * iy * ix * *pf;
+				v = kf * idf + kmu * (v + *pr);
+				pf += sz;
+				pr += sz;
 			}
+			if (dot) acc += uc * v;
 			*po = v;
 			uzm = uc;
 			uc = uzp;
@@ -178,23 +177,30 @@ march_apply_kernel(FluidOps o, const double* __restrict__ u, double* __restrict_
 	}
 }
 
+// Planes per thread and grid of the marching operator.
+struct March {
+	dim3 grid;
+	int zrun = kMarchZ;
+	int blocks() const { return (int) (grid.x * grid.y * grid.z); }
+};
+
 template <int OP>
-void launch_march_dims(const FluidOps& o, dim3 grid, const double* u, double* out, double* dot, const double* r,
-                       double wa, double wb, cudaStream_t s)
+void launch_march_dims(const FluidOps& o, const March& m, const double* u, double* out, double* dot, const double* f,
+                       const double* rhs0, double kf, double kmu, cudaStream_t s)
 {
-	if (o.dims == 3) march_apply_kernel<OP, 3><<<grid, dim3(kMarchX, kMarchY), 0, s>>>(o, u, out, dot, r, wa, wb);
-	else march_apply_kernel<OP, 2><<<grid, dim3(kMarchX, kMarchY), 0, s>>>(o, u, out, dot, r, wa, wb);
+	const dim3 block(kMarchX, kMarchY);
+	if (o.dims == 3) march_apply_kernel<OP, 3><<<m.grid, block, 0, s>>>(o, u, out, dot, m.zrun, f, rhs0, kf, kmu);
+	else march_apply_kernel<OP, 2><<<m.grid, block, 0, s>>>(o, u, out, dot, m.zrun, f, rhs0, kf, kmu);
 }
 
-void launch_march(const FluidOps& o, int op, dim3 grid, const double* u, double* out, double* dot, cudaStream_t s,
-                  const double* r = nullptr, double wa = 0.0, double wb = 0.0)
+void launch_march(const FluidOps& o, int op, const March& m, const double* u, double* out, double* dot, cudaStream_t s,
+                  const double* f = nullptr, const double* rhs0 = nullptr, double kf = 0.0, double kmu = 0.0)
 {
 	switch (op) {
-	case 0: launch_march_dims<0>(o, grid, u, out, dot, r, wa, wb, s); break;
-	case 1: launch_march_dims<1>(o, grid, u, out, dot, r, wa, wb, s); break;
-	case 2: launch_march_dims<2>(o, grid, u, out, dot, r, wa, wb, s); break;
-	case 3: launch_march_dims<3>(o, grid, u, out, dot, r, wa, wb, s); break;
-	default: launch_march_dims<4>(o, grid, u, out, dot, r, wa, wb, s); break;
+	case 0: launch_march_dims<0>(o, m, u, out, dot, f, rhs0, kf, kmu, s); break;
+	case 1: launch_march_dims<1>(o, m, u, out, dot, f, rhs0, kf, kmu, s); break;
+	case 2: launch_march_dims<2>(o, m, u, out, dot, f, rhs0, kf, kmu, s); break;
+	default: launch_march_dims<3>(o, m, u, out, dot, f, rhs0, kf, kmu, s); break;
 	}
 }
 
@@ -299,16 +305,6 @@ __global__ void __launch_bounds__(kSumThreads) sum_kernel(const double* __restri
 	if (threadIdx.x == 0) *out = t;
 }
 
-// rhs = k I~ f + k mu (L u + rhs0): the right-hand side of the solve
-// (diffusion.h:51-53: gemv(1, L, u, 1, rhs), then gemv(k, I~, f, k mu, rhs)).
-__global__ void __launch_bounds__(kFluidThreads)
-rhs_kernel(long long n, double k, double kmu, const double* __restrict__ lu, const double* __restrict__ rhs0,
-           const double* __restrict__ idf, double* __restrict__ b)
-{
-	for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x)
-		b[i] = k * idf[i] + kmu * (lu[i] + rhs0[i]);
-}
-
 // Start of the loop: x = 0, d = M^-1 r (dinv: the reciprocal diagonal),
 // partials of r . d and d . d.
 __global__ void __launch_bounds__(kFluidThreads)
@@ -329,7 +325,10 @@ start_kernel(long long n, const double* __restrict__ r, const double* __restrict
 }
 
 // Device scalars of the loop (sc): [0] delta = r . M^-1 r, [1] nu = d . H d,
-// [2] |d|^2, [3] alpha, [4] beta, [5] stop (1 when nu fell below tol^2).
+// [2] |d|^2, [3] alpha, [4] beta, [5] stop (0 running, else a Stop), [6]
+// finished iterations (Chebyshev loop).
+constexpr int kScalars = 8;
+enum Stop { kBailOut = 1, kConverged = 2, kLimit = 3 };    // nu below tol^2; |d| <= tol; max_iterations
 
 // nu from its partials; alpha = delta / nu, or stop (pcg.h:23-31).
 __global__ void __launch_bounds__(kSumThreads) alpha_kernel(const double* __restrict__ partial, int n, double tol2,
@@ -373,31 +372,6 @@ update_kernel(long long n, const double* __restrict__ sc, const double* __restri
 	block_partial(a, rq);
 }
 
-// x += alpha d, r -= alpha q (the Chebyshev preconditioner and the r . z
-// partials follow in the operator kernel).  Does nothing once the loop has
-// stopped.
-__global__ void __launch_bounds__(kFluidThreads, 8)
-update_xr_kernel(long long n, const double* __restrict__ sc, const double* __restrict__ d,
-                 const double* __restrict__ q, double* __restrict__ x, double* __restrict__ r)
-{
-	if (sc[5] != 0.0) return;
-	const double alpha = sc[3];
-	for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-		x[i] += alpha * d[i];
-		r[i] = r[i] - alpha * q[i];
-	}
-}
-
-// |d|^2 partials (the start of the loop under the Chebyshev preconditioner).
-__global__ void __launch_bounds__(kFluidThreads)
-norm_kernel(long long n, const double* __restrict__ d, double* __restrict__ dd)
-{
-	double a = 0.0;
-	for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x)
-		a += d[i] * d[i];
-	block_partial(a, dd);
-}
-
 // d = q + beta d; partial sums of d . d.
 __global__ void __launch_bounds__(kFluidThreads)
 direction_kernel(long long n, const double* __restrict__ sc, const double* __restrict__ q, double* __restrict__ d,
@@ -412,6 +386,492 @@ direction_kernel(long long n, const double* __restrict__ sc, const double* __res
 		a += v * v;
 	}
 	block_partial(a, dd);
+}
+
+// ------------------------------------------ Chebyshev-preconditioned loop
+// One iteration is two kernels, each a tile of (x, y) columns marched along
+// z, with the plane that the x and y neighbours come from in shared memory
+// (two buffers, one barrier per plane) and the z neighbours in registers:
+//   direction_apply_kernel  d' = z + beta d, x += alpha d, q = H d' and the
+//                           sums of d' . q and d' . d'; the stopping tests'
+//                           outcome also goes to the host's memory
+//   polynomial_kernel       r' = r - alpha q, z = p(H) r' (the three steps
+//                           s <- w_i r' - H s of the degree-4 polynomial in
+//                           one pass, on a halo of 3) and the sum of r' . z
+// Both write r and d to the other of two buffers: neighbouring blocks still
+// read the old values on their halos.  The last block to finish adds up the
+// blocks' partial sums in block order (so every run has the same bits) and
+// forms alpha or beta and the stopping tests there.  HBM traffic per face and
+// iteration: 48 + 32 bytes (one kernel per operator product, update and
+// direction moved 152).  The products use fused multiply-adds with lambda
+// folded into the coefficients; the operators themselves
+// (march_apply_kernel) keep the reference's operation order.
+
+// Index of an extended coordinate on an axis: wrapped on a periodic axis, -1
+// outside a wall.
+__device__ __forceinline__ int fold_index(const AxisOps& a, int v)
+{
+	if (a.periodic) {
+		v %= a.P;
+		return v < 0 ? v + a.P : v;
+	}
+	return v >= 0 && v < a.P ? v : -1;
+}
+
+// One axis' coefficients at index v of -lambda L and I~; all 0 for v < 0
+// (nothing of the grid there: such a face stays 0 through every step) and for
+// an axis the run does not have, but for id = 1 at v = 0.
+struct AxisCoef { double lo, diag, hi, id; };
+
+__device__ __forceinline__ AxisCoef axis_coef(const AxisOps& a, bool present, double lambda, int v)
+{
+	if (v < 0) return {0.0, 0.0, 0.0, 0.0};
+	if (!present) return {0.0, 0.0, 0.0, 1.0};
+	return {-lambda * __ldg(a.lo + v), -lambda * __ldg(a.diag + v), -lambda * __ldg(a.hi + v), __ldg(a.id + v)};
+}
+
+// Sums over the block, in a fixed order: valid in thread 0.
+template <int NT, int N>
+__device__ __forceinline__ void block_sums(double* v)
+{
+	__shared__ double red[N][NT / 32];
+#pragma unroll
+	for (int q = 0; q < N; ++q) {
+		for (int s = 16; s > 0; s >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], s);
+		if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = v[q];
+	}
+	__syncthreads();
+	if (threadIdx.x == 0) {
+#pragma unroll
+		for (int q = 0; q < N; ++q) {
+			double t = 0.0;
+			for (int w = 0; w < NT / 32; ++w) t += red[q][w];
+			v[q] = t;
+		}
+	}
+	__syncthreads();
+}
+
+// Leaves the block's N sums in part and returns true in every thread of the
+// last block to do so, with the totals over all blocks in v of thread 0.
+// done: zero before the launch and after it.
+template <int NT, int N>
+__device__ __forceinline__ bool grid_sums(double* v, double* part, unsigned* done)
+{
+	__shared__ bool last;
+	const int nblocks = gridDim.x * gridDim.y * gridDim.z;
+	block_sums<NT, N>(v);
+	if (threadIdx.x == 0) {
+		const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+#pragma unroll
+		for (int q = 0; q < N; ++q) __stcg(part + (size_t) q * nblocks + b, v[q]);
+		__threadfence();
+		last = atomicAdd(done, 1u) == (unsigned) nblocks - 1u;
+	}
+	__syncthreads();
+	if (!last) return false;
+	__threadfence();
+#pragma unroll
+	for (int q = 0; q < N; ++q) {
+		v[q] = 0.0;
+		for (int b = threadIdx.x; b < nblocks; b += NT) v[q] += __ldcg(part + (size_t) q * nblocks + b);
+	}
+	block_sums<NT, N>(v);
+	if (threadIdx.x == 0) *done = 0u;
+	return true;
+}
+
+// Plane p on the z axis, at most three planes past its ends: wrapped on a
+// periodic axis, -1 outside a wall.
+__device__ __forceinline__ int fold_plane(const AxisOps& a, int p)
+{
+	if (p < 0) return a.periodic ? p + a.P : -1;
+	if (p >= a.P) return a.periodic ? p - a.P : -1;
+	return p;
+}
+
+// Whether the faces lo .. hi of an axis all carry the interior's coefficients
+// and exist: no wall in reach.
+__device__ __forceinline__ bool alike(const AxisOps& a, int lo, int hi)
+{
+	return a.periodic || (lo >= 1 && hi <= a.P - 2);
+}
+
+// H at a face in two parts: partial() without the plane above (c the face's
+// value, then its neighbours left, right, in the rows before and after and in
+// the plane below), and the weight top() of the plane above.  Row and plane
+// index the block's tables.  Three forms, by what walls a block can reach:
+// none (one weight for the face and one for its six neighbours, and no
+// coefficient to load),
+struct UniformH {
+	static constexpr bool uniform = true;       // every column and plane in reach is on the grid
+	double centre, side;
+	__device__ __forceinline__ UniformH(const FluidOps& o, const AxisCoef& cx, const AxisCoef*, const AxisCoef*)
+		: centre(1.0 + o.dims * cx.diag), side(cx.lo) {}
+	__device__ __forceinline__ double partial(int, int, double c, double xm, double xp, double ym, double yp, double zm) const
+	{
+		return __fma_rn(centre, c, side * (((xm + xp) + (ym + yp)) + zm));
+	}
+	__device__ __forceinline__ double top(int, int) const { return side; }
+};
+
+// walls along y only (a channel),
+struct WallYH {
+	static constexpr bool uniform = false;
+	double centre, side;
+	const AxisCoef* yt;
+	__device__ __forceinline__ WallYH(const FluidOps&, const AxisCoef& cx, const AxisCoef* y, const AxisCoef*)
+		: centre(1.0 + 2.0 * cx.diag), side(cx.lo), yt(y) {}
+	__device__ __forceinline__ double partial(int row, int, double c, double xm, double xp, double ym, double yp,
+	                                          double zm) const
+	{
+		const AxisCoef y = yt[row];
+		const double xz = __fma_rn(centre, c, side * ((xm + xp) + zm));
+		return __fma_rn(y.id, xz, __fma_rn(y.hi, yp, __fma_rn(y.lo, ym, y.diag * c)));
+	}
+	__device__ __forceinline__ double top(int row, int) const { return side * yt[row].id; }
+};
+
+// and any.
+struct GeneralH {
+	static constexpr bool uniform = false;
+	AxisCoef x;
+	const AxisCoef *yt, *zt;
+	__device__ __forceinline__ GeneralH(const FluidOps&, const AxisCoef& cx, const AxisCoef* y, const AxisCoef* z)
+		: x(cx), yt(y), zt(z) {}
+	__device__ __forceinline__ double partial(int row, int plane, double c, double xm, double xp, double ym, double yp,
+	                                          double zm) const
+	{
+		const AxisCoef y = yt[row], z = zt[plane];
+		const double ax = __fma_rn(x.hi, xp, __fma_rn(x.lo, xm, (x.id + x.diag) * c));
+		const double ay = __fma_rn(y.hi, yp, __fma_rn(y.lo, ym, y.diag * c));
+		const double az = __fma_rn(z.lo, zm, z.diag * c);
+		return __fma_rn(x.id * y.id, az, z.id * __fma_rn(x.id, ay, y.id * ax));
+	}
+	__device__ __forceinline__ double top(int row, int plane) const { return x.id * yt[row].id * zt[plane].hi; }
+};
+
+// The coefficients of `count` faces from `first` on along an axis.
+__device__ __forceinline__ void fill_table(const FluidOps& o, int axis, int first, int count, AxisCoef* t)
+{
+	for (int i = threadIdx.x; i < count; i += blockDim.x)
+		t[i] = axis_coef(o.ax[axis], axis < o.dims, o.lambda, fold_index(o.ax[axis], first + i));
+}
+
+// Time of one step of polynomial_kernel's wide tile over the small tile's
+// (from the solves timed above).
+constexpr double kWideStep = 1.5;
+
+// Longest run of planes per block (bounds the tables along z).
+constexpr int kMaxRun = 64;
+
+// direction_apply_kernel's tile: 64 x 8 columns, 256 threads with two
+// neighbouring rows each; the first 144 threads also hold one column each of
+// the halo.  Bound by HBM: 48 bytes per face, the next plane's z, d and x
+// loaded a plane ahead.  512 x 256 x 512 faces: 551 us, 5.85 TB/s (operator,
+// half the update and the direction as passes of their own: 336 + 237 + 241
+// us).  At most three CTAs per SM: with four (64 registers) it spills, 2 to 5 %
+// slower.
+constexpr int kDirX = 64, kDirY = 8, kDirRows = 2, kDirThreads = 256, kDirBlocks = 3;
+constexpr int kDirStride = kDirX + 2;
+
+__global__ void __launch_bounds__(kDirThreads, kDirBlocks)
+direction_apply_kernel(FluidOps o, double* __restrict__ sc, const double* __restrict__ z,
+                       const double* __restrict__ dold, double* __restrict__ dnew, double* __restrict__ x,
+                       double* __restrict__ q, double* __restrict__ part, unsigned* __restrict__ done, int zrun,
+                       int first, double tol, int max_iterations, double* __restrict__ host)
+{
+	if (sc[5] != 0.0) return;
+	__shared__ double plane[2][(kDirY + 2) * kDirStride];
+	__shared__ AxisCoef zt[kMaxRun];
+	__shared__ AxisCoef yt[kDirY];
+	const double alpha = sc[3], beta = sc[4];
+	const int P0 = o.ax[0].P, P1 = o.ax[1].P;
+	const int tx = threadIdx.x % kDirX, ty = threadIdx.x / kDirX;
+	const int x0 = blockIdx.x * kDirX, y0 = blockIdx.y * kDirY;
+	const int k0 = blockIdx.z * zrun, k1 = min(k0 + zrun, o.ax[2].P);
+	const int sz = P0 * P1;
+
+	const int gi = fold_index(o.ax[0], x0 + tx);
+	int off[kDirRows];          // the column's offset in a plane, -1 outside
+	bool own[kDirRows];         // this block writes it
+#pragma unroll
+	for (int c = 0; c < kDirRows; ++c) {
+		const int y = y0 + ty * kDirRows + c;
+		const int gj = fold_index(o.ax[1], y);
+		off[c] = gi >= 0 && gj >= 0 ? gi + gj * P0 : -1;
+		own[c] = x0 + tx < P0 && y < P1;
+	}
+	// halo columns: the rows above and below, then the columns left and right
+	int hoff = -1, hslot = -1;
+	if (threadIdx.x < 2 * kDirX + 2 * kDirY) {
+		const int t = threadIdx.x, h = t - 2 * kDirX;
+		const int ex = h < 0 ? t % kDirX : (h < kDirY ? -1 : kDirX);
+		const int ey = h < 0 ? (t < kDirX ? -1 : kDirY) : h % kDirY;
+		hslot = (ey + 1) * kDirStride + ex + 1;
+		const int hi = fold_index(o.ax[0], x0 + ex), hj = fold_index(o.ax[1], y0 + ey);
+		if (hi >= 0 && hj >= 0) hoff = hi + hj * P0;
+	}
+	const int slot = (ty * kDirRows + 1) * kDirStride + tx + 1;
+	double sums[2] = {0.0, 0.0};
+
+	auto march = [&](const auto& H) {
+		constexpr bool uniform = std::decay_t<decltype(H)>::uniform;
+		// loads of one plane, a plane ahead of their use
+		double zv[kDirRows], dv[kDirRows], xv[kDirRows], hz = 0.0, hd = 0.0;
+		auto fetch = [&](int p, bool inner) {
+			const int g = fold_plane(o.ax[2], p);
+			const double *zp = z + (long long) g * sz, *dp = dold + (long long) g * sz;
+#pragma unroll
+			for (int c = 0; c < kDirRows; ++c) {
+				const bool on = uniform || (g >= 0 && off[c] >= 0);
+				zv[c] = on ? __ldg(zp + off[c]) : 0.0;
+				dv[c] = on && !first ? __ldg(dp + off[c]) : 0.0;
+				xv[c] = inner && own[c] && !first ? x[g * sz + off[c]] : 0.0;
+			}
+			if (hslot >= 0) {
+				const bool hon = uniform || (g >= 0 && hoff >= 0);
+				hz = hon ? __ldg(zp + hoff) : 0.0;
+				hd = hon && !first ? __ldg(dp + hoff) : 0.0;
+			}
+		};
+		// plane k of d': registers and shared buffer k & 1; d' and x written
+		auto take = [&](int k, bool inner, double* v) {
+			double* buf = plane[k & 1];
+#pragma unroll
+			for (int c = 0; c < kDirRows; ++c) {
+				v[c] = __fma_rn(beta, dv[c], zv[c]);
+				buf[slot + c * kDirStride] = v[c];
+				if (inner && own[c]) {
+					dnew[k * sz + off[c]] = v[c];
+					x[k * sz + off[c]] = __fma_rn(alpha, dv[c], xv[c]);
+				}
+			}
+			if (hslot >= 0) buf[hslot] = __fma_rn(beta, hd, hz);
+		};
+		double vm[kDirRows], vc[kDirRows], vn[kDirRows];
+		fetch(k0 - 1, false);
+#pragma unroll
+		for (int c = 0; c < kDirRows; ++c) vm[c] = __fma_rn(beta, dv[c], zv[c]);
+		fetch(k0, true);
+		take(k0, true, vc);
+		fetch(k0 + 1, k0 + 1 < k1);
+		for (int k = k0; k < k1; ++k) {
+			__syncthreads();            // plane k is complete; every read of plane k - 1 is done
+			take(k + 1, k + 1 < k1, vn);
+			if (k + 1 < k1) fetch(k + 2, k + 2 < k1);
+			const double* buf = plane[k & 1];
+#pragma unroll
+			for (int c = 0; c < kDirRows; ++c) {
+				const int at = slot + c * kDirStride;
+				const double ym = c > 0 ? vc[c - 1] : buf[at - kDirStride];
+				const double yp = c + 1 < kDirRows ? vc[c + 1] : buf[at + kDirStride];
+				const int row = ty * kDirRows + c;
+				const double h = __fma_rn(H.top(row, k - k0), vn[c],
+				                          H.partial(row, k - k0, vc[c], buf[at - 1], buf[at + 1], ym, yp, vm[c]));
+				if (own[c]) {
+					q[k * sz + off[c]] = h;
+					sums[0] = __fma_rn(vc[c], h, sums[0]);
+					sums[1] = __fma_rn(vc[c], vc[c], sums[1]);
+				}
+			}
+#pragma unroll
+			for (int c = 0; c < kDirRows; ++c) { vm[c] = vc[c]; vc[c] = vn[c]; }
+		}
+	};
+	const AxisCoef cx = axis_coef(o.ax[0], true, o.lambda, gi);
+	if (alike(o.ax[0], x0 - 1, x0 + kDirX) && alike(o.ax[1], y0 - 1, y0 + kDirY) && alike(o.ax[2], k0 - 1, k1)) {
+		march(UniformH(o, cx, yt, zt));
+	} else {
+		fill_table(o, 1, y0, kDirY, yt);
+		fill_table(o, 2, k0, k1 - k0, zt);
+		if (alike(o.ax[0], x0 - 1, x0 + kDirX) && alike(o.ax[2], k0 - 1, k1))
+			march(WallYH(o, cx, yt, zt));
+		else
+			march(GeneralH(o, cx, yt, zt));     // the first barrier comes before the tables are read
+	}
+	if (!grid_sums<kDirThreads, 2>(sums, part, done) || threadIdx.x != 0) return;
+	// the loop test of pcg.h:21, then alpha or the bail-out of pcg.h:23-31
+	sc[1] = sums[0];
+	sc[2] = sums[1];
+	if (!(sqrt(sums[1]) > tol)) sc[5] = kConverged;
+	else if (sc[6] >= (double) max_iterations) sc[5] = kLimit;
+	else if (fabs(sums[0]) < tol * tol) sc[5] = kBailOut;
+	else sc[3] = sc[0] / sums[0];
+	host[0] = sc[5];
+	host[1] = sc[6];
+}
+
+// polynomial_kernel's tile: EX x TY * ROWS columns, of which the inner ones (a
+// halo of 3) are the block's own, EX x TY threads with ROWS neighbouring rows
+// each.  At step p the block takes plane p of r' and finishes the first
+// step's plane p - 1, the second's p - 2 and the third's p - 3, each from the
+// part that was formed as soon as the planes below were there: what follows
+// the barrier is three independent parts.  Columns and planes at the rim of
+// the halo hold values that nothing inside uses.
+template <int EX_, int TY_, int ROWS_, int BLOCKS_>
+struct PolyTile {
+	static constexpr int EX = EX_, TY = TY_, ROWS = ROWS_, BLOCKS = BLOCKS_, HALO = 3;
+	static constexpr int EY = TY * ROWS, X = EX - 2 * HALO, Y = EY - 2 * HALO, THREADS = EX * TY;
+	static constexpr int PLANE = EX * EY, BYTES = 6 * PLANE * (int) sizeof(double);
+	static_assert(THREADS % 32 == 0, "whole warps");
+};
+// Two thirds of the wide tile's columns are the block's own, half of the small
+// tile's; the small one has three times the blocks.  512 x 256 x 512 faces
+// 20.2 ms a solve against 23.4 ms, 256 x 128 x 256 3.43 against 3.57, 128^3
+// 1.11 against 1.09, 117 x 234 x 117 1.85 against 1.76, 64^3 0.49 against 0.46.
+using PolyWide = PolyTile<64, 8, 3, 1>;
+using PolySmall = PolyTile<32, 16, 1, 2>;
+
+struct ChebWeights { double w[4]; };
+
+template <typename T>
+__global__ void __launch_bounds__(T::THREADS, T::BLOCKS)
+polynomial_kernel(FluidOps o, double* __restrict__ sc, const double* __restrict__ r, const double* __restrict__ q,
+                  double* __restrict__ rnew, double* __restrict__ z, double* __restrict__ part,
+                  unsigned* __restrict__ done, int zrun, int first, ChebWeights cw)
+{
+	if (sc[5] != 0.0) return;
+	extern __shared__ double poly_planes[];     // r', first and second step: two buffers each
+	__shared__ AxisCoef zt[kMaxRun + 2 * T::HALO];
+	__shared__ AxisCoef yt[T::EY];
+	const double alpha = sc[3];
+	const int P0 = o.ax[0].P, P1 = o.ax[1].P;
+	const int tx = threadIdx.x % T::EX, ty = threadIdx.x / T::EX;
+	const int ex0 = (int) blockIdx.x * T::X - T::HALO, ey0 = (int) blockIdx.y * T::Y - T::HALO;
+	const int k0 = blockIdx.z * zrun, k1 = min(k0 + zrun, o.ax[2].P);
+	const int sz = P0 * P1;
+
+	const int gi = fold_index(o.ax[0], ex0 + tx);
+	int off[T::ROWS];
+	bool own[T::ROWS];
+#pragma unroll
+	for (int c = 0; c < T::ROWS; ++c) {
+		const int ey = ty * T::ROWS + c, y = ey0 + ey;
+		const int gj = fold_index(o.ax[1], y);
+		off[c] = gi >= 0 && gj >= 0 ? gi + gj * P0 : -1;
+		own[c] = tx >= T::HALO && tx < T::HALO + T::X && ex0 + tx < P0 && ey >= T::HALO &&
+		         ey < T::HALO + T::Y && y < P1;
+	}
+	const int slot = ty * T::ROWS * T::EX + tx;
+	const int left = tx > 0 ? -1 : 0, right = tx + 1 < T::EX ? 1 : 0;
+	const int above = ty > 0 ? -T::EX : 0, below = ty + 1 < T::TY ? T::EX : 0;
+	double sums[1] = {0.0};
+
+	auto march = [&](const auto& H) {
+		constexpr bool uniform = std::decay_t<decltype(H)>::uniform;
+		double rv[T::ROWS], qv[T::ROWS];
+		auto fetch = [&](int p) {
+			const int g = fold_plane(o.ax[2], p);
+			const double *rp = r + (long long) g * sz, *qp = q + (long long) g * sz;
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c) {
+				const bool on = uniform || (g >= 0 && off[c] >= 0);
+				rv[c] = on ? __ldg(rp + off[c]) : 0.0;
+				qv[c] = on && !first ? __ldg(qp + off[c]) : 0.0;
+			}
+		};
+		// the part of w v - ws H s at plane k that does not need plane k + 1, for
+		// this thread's columns: s and sm its values at planes k and k - 1, buf the
+		// shared copy of plane k; above() adds the rest
+		auto below_part = [&](const double* buf, int k, double w, double ws, const double* v, const double* s,
+		                      const double* sm, double* out) {
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c) {
+				const int at = slot + c * T::EX;
+				const double ym = c > 0 ? s[c - 1] : buf[at + above];
+				const double yp = c + 1 < T::ROWS ? s[c + 1] : buf[at + below];
+				const double h = H.partial(ty * T::ROWS + c, k - k0 + T::HALO, s[c], buf[at + left], buf[at + right], ym,
+				                           yp, sm[c]);
+				out[c] = __fma_rn(w, v[c], -ws * h);
+			}
+		};
+		auto add_above = [&](int k, double ws, const double* part_, const double* sp, double* out) {
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c)
+				out[c] = __fma_rn(-ws * H.top(ty * T::ROWS + c, k - k0 + T::HALO), sp[c], part_[c]);
+		};
+		// r' at planes p - 1 .. p - 3, the first step at p - 2, the second at p -
+		// 3, and the three steps' parts at p - 1, p - 2, p - 3
+		double v1[T::ROWS] = {}, v2[T::ROWS] = {}, v3[T::ROWS] = {}, am[T::ROWS] = {}, bm[T::ROWS] = {};
+		double pa[T::ROWS] = {}, pb[T::ROWS] = {}, pz[T::ROWS] = {};
+		fetch(k0 - T::HALO);
+		for (int p = k0 - T::HALO; p < k1 + T::HALO; ++p) {
+			double v0[T::ROWS], a1[T::ROWS], b2[T::ROWS], out[T::ROWS];
+			double* buf = poly_planes + (p & 1) * (3 * T::PLANE);
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c) v0[c] = __fma_rn(-alpha, qv[c], rv[c]);
+			if (p + 1 < k1 + T::HALO) fetch(p + 1);
+			add_above(max(p - 1, k0 - T::HALO), cw.w[0], pa, v0, a1);
+			add_above(max(p - 2, k0 - T::HALO), 1.0, pb, a1, b2);
+			add_above(max(p - 3, k0 - T::HALO), 1.0, pz, b2, out);
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c) {
+				const int at = slot + c * T::EX;
+				buf[at] = v0[c];
+				buf[T::PLANE + at] = a1[c];
+				buf[2 * T::PLANE + at] = b2[c];
+			}
+			if (p - 3 >= k0) {
+#pragma unroll
+				for (int c = 0; c < T::ROWS; ++c)
+					if (own[c]) {
+						const int at = (p - 3) * sz + off[c];
+						rnew[at] = v3[c];
+						z[at] = out[c];
+						sums[0] = __fma_rn(v3[c], out[c], sums[0]);
+					}
+			}
+			__syncthreads();        // this step's planes are complete; the other buffer's reads are done
+			below_part(buf, p, cw.w[1], cw.w[0], v0, v0, v1, pa);
+			below_part(buf + T::PLANE, max(p - 1, k0 - T::HALO), cw.w[2], 1.0, v1, a1, am, pb);
+			below_part(buf + 2 * T::PLANE, max(p - 2, k0 - T::HALO), cw.w[3], 1.0, v2, b2, bm, pz);
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c) {
+				v3[c] = v2[c]; v2[c] = v1[c]; v1[c] = v0[c];
+				am[c] = a1[c];
+				bm[c] = b2[c];
+			}
+		}
+	};
+	const AxisCoef cx = axis_coef(o.ax[0], true, o.lambda, gi);
+	if (alike(o.ax[0], ex0, ex0 + T::EX - 1) && alike(o.ax[1], ey0, ey0 + T::EY - 1) &&
+	    alike(o.ax[2], k0 - T::HALO, k1 + T::HALO - 1)) {
+		march(UniformH(o, cx, yt, zt));
+	} else {
+		fill_table(o, 1, ey0, T::EY, yt);
+		fill_table(o, 2, k0 - T::HALO, k1 - k0 + 2 * T::HALO, zt);
+		__syncthreads();
+		if (alike(o.ax[0], ex0, ex0 + T::EX - 1) && alike(o.ax[2], k0 - T::HALO, k1 + T::HALO - 1))
+			march(WallYH(o, cx, yt, zt));
+		else
+			march(GeneralH(o, cx, yt, zt));
+	}
+	if (!grid_sums<T::THREADS, 1>(sums, part, done) || threadIdx.x != 0) return;
+	if (first) {
+		sc[0] = sums[0];            // pcg.h:14-18: delta = r . d
+	} else {
+		sc[4] = sums[0] / sc[0];    // pcg.h:36-39: beta = delta' / delta
+		sc[0] = sums[0];
+		sc[6] += 1.0;
+	}
+}
+
+// Planes per block of a tile kernel and the cost that comes with them: rounds
+// of work over the resident blocks, a round being the block's planes, the
+// halo planes that it recomputes and about three planes' time to start and
+// finish.
+struct Run { int planes; long long cost; };
+
+Run pick_run(long long tiles, int planes, int halo, long long resident)
+{
+	Run best{1, -1};
+	for (int run = 1; run <= std::min(planes, kMaxRun); ++run) {
+		const long long blocks = tiles * ((planes + run - 1) / run);
+		const long long cost = ((blocks + resident - 1) / resident) * (run + 2 * halo + 3);
+		if (best.cost < 0 || cost <= best.cost) best = {run, cost};
+	}
+	return best;
 }
 
 // out = u + x
@@ -467,21 +927,143 @@ ibk_status cuda_fail(cudaError_t e, const char* what)
 
 using namespace ibk;
 
+// Iterations queued beyond the one whose stopping test the host waits for.
+// The test runs on the device and the kernels of a stopped loop return at
+// once, so a few iterations too many cost a few microseconds, while waiting
+// for every test before queueing more would leave the GPU idle for the round
+// trip (about 20 us of each iteration; a 64^3 grid's takes about that long).
+constexpr int kLookAhead = 2;
+
 struct ibk_diffusion_s {
 	int device = 0;
 	FluidOps ops{};
 	double mu = 0.0, timestep = 0.0, tolerance = 0.0;
 	int max_iterations = 0;
 	double* coef = nullptr;        // per axis: lo, diag, hi, id (4 P_d doubles)
-	double* work = nullptr;        // b, r, d, q, x, diag, tmp, tmp2 (8 size doubles)
+	double* work = nullptr;        // 8 arrays of size doubles (see Work)
 	int precond = IBK_PRECOND_CHEBYSHEV;
 	double cheb_w[4] = {};         // chebw<4> on the Gershgorin interval
 	double bounds[2] = {};         // that interval (lower, upper)
-	double* partial = nullptr;     // partial sums: max(march blocks, kFluidBlocks) + kFluidBlocks
-	dim3 march_grid;               // march_apply_kernel's grid
-	int march_blocks = 0;
-	double* scalars = nullptr;     // device scalars of the loop (see alpha_kernel)
+	double* partial = nullptr;     // the blocks' partial sums
+	int first_partials = 0;        // room for the first of two sets
+	March march;                   // march_apply_kernel's grid
+	dim3 dir_grid, poly_grid;      // grids and planes per block of the Chebyshev loop's kernels
+	int dir_run = 1, poly_run = 1;
+	bool poly_wide = true;
+	double* scalars = nullptr;     // device scalars of the loop, then the kernels' counter of finished blocks
+	double* host_tests = nullptr;                   // pinned: stop and iterations of each look-ahead slot
+	cudaEvent_t tested[kLookAhead + 1] = {};        // the kernel that writes each slot
 };
+
+namespace {
+
+// The right-hand side of the solve: k I~ f + k mu (L u + rhs).
+void launch_rhs(const ibk_diffusion_s& d, double gamma, const double* u, const double* rhs, const double* f, double* b,
+                cudaStream_t s)
+{
+	const double k = gamma * d.timestep;
+	launch_march(d.ops, 3, d.march, u, b, nullptr, s, f, rhs, k, k * d.mu);
+}
+
+const char* const kNoConvergence = "diffusion solve did not converge within max_iterations";
+
+// The loop with the Chebyshev preconditioner (two kernels an iteration).
+ibk_status step_chebyshev(ibk_diffusion_s& d, double gamma, const double* u, const double* rhs, const double* f,
+                          double* out, int* iterations, cudaStream_t s)
+{
+	const long long n = d.ops.size;
+	double* r[2] = {d.work, d.work + n};
+	double* dv[2] = {d.work + 2 * n, d.work + 3 * n};
+	double *q = d.work + 4 * n, *x = d.work + 6 * n, *z = d.work + 7 * n;
+	double* sc = d.scalars;
+	unsigned* done = reinterpret_cast<unsigned*>(sc + kScalars);
+	ChebWeights cw;
+	std::copy(d.cheb_w, d.cheb_w + 4, cw.w);
+	cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(double) * (kScalars + 1), s);
+	if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+	launch_rhs(d, gamma, u, rhs, f, r[0], s);
+	const auto polynomial = [&](const double* rin, double* rout, int first) {
+		if (d.poly_wide)
+			polynomial_kernel<PolyWide><<<d.poly_grid, PolyWide::THREADS, PolyWide::BYTES, s>>>(
+				d.ops, sc, rin, q, rout, z, d.partial, done, d.poly_run, first, cw);
+		else
+			polynomial_kernel<PolySmall><<<d.poly_grid, PolySmall::THREADS, PolySmall::BYTES, s>>>(
+				d.ops, sc, rin, q, rout, z, d.partial, done, d.poly_run, first, cw);
+	};
+	polynomial(r[0], r[1], 1);
+	ibk_status st = check_launch("diffusion set-up kernels");
+	if (st != IBK_OK) return st;
+	const double* seen = nullptr;          // the test that stopped the loop
+	for (long long it = 0; !seen; ++it) {
+		const int a = (int) (it & 1), slot = (int) (it % (kLookAhead + 1));
+		direction_apply_kernel<<<d.dir_grid, kDirThreads, 0, s>>>(d.ops, sc, z, dv[a], dv[a ^ 1], x, q, d.partial, done,
+		                                                          d.dir_run, it == 0, d.tolerance, d.max_iterations,
+		                                                          d.host_tests + 2 * slot);
+		if ((e = cudaEventRecord(d.tested[slot], s)) != cudaSuccess) return cuda_fail(e, "diffusion residual read");
+		polynomial(r[a ^ 1], r[a], 0);
+		if ((st = check_launch("diffusion iteration kernels")) != IBK_OK) return st;
+		if (it < kLookAhead) continue;
+		const int back = (int) ((it - kLookAhead) % (kLookAhead + 1));
+		if ((e = cudaEventSynchronize(d.tested[back])) != cudaSuccess) return cuda_fail(e, "diffusion residual read");
+		if (d.host_tests[2 * back] != 0.0) seen = d.host_tests + 2 * back;
+	}
+	// the queued iterations find the loop stopped; they are over before the
+	// next call may start another on this handle's scalars
+	if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "diffusion residual read");
+	if (iterations) *iterations = (int) seen[1];
+	if (seen[0] == kLimit) return set_error(IBK_ERR_DEVICE_CHECK, kNoConvergence);
+	finish_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, u, x, out);
+	return check_launch("finish_kernel");
+}
+
+// The loop with the Jacobi preconditioner.
+ibk_status step_jacobi(ibk_diffusion_s& d, double gamma, const double* u, const double* rhs, const double* f,
+                       double* out, int* iterations, cudaStream_t s)
+{
+	const long long n = d.ops.size;
+	double *r = d.work, *dv = d.work + 2 * n, *q = d.work + 4 * n, *diag = d.work + 5 * n, *x = d.work + 6 * n;
+	double* pa = d.partial;
+	double* pb = d.partial + d.first_partials;
+	double* sc = d.scalars;
+	cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(double) * kScalars, s);
+	if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+	launch_rhs(d, gamma, u, rhs, f, r, s);
+	start_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, r, diag, x, dv, pa, pb);
+	sum_kernel<<<1, kSumThreads, 0, s>>>(pa, kFluidBlocks, sc + 0);
+	sum_kernel<<<1, kSumThreads, 0, s>>>(pb, kFluidBlocks, sc + 2);
+	ibk_status st = check_launch("diffusion set-up kernels");
+	if (st != IBK_OK) return st;
+	const double tol = d.tolerance;
+	int it = 0;
+	double hs[6];
+	for (;;) {
+		// the loop test of pcg.h:21 (|d| > tol) and its bail-out, read back once
+		// per iteration; alpha and beta stay on the device
+		e = cudaMemcpyAsync(hs, sc, sizeof(double) * 6, cudaMemcpyDeviceToHost, s);
+		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+		if (e != cudaSuccess) return cuda_fail(e, "diffusion residual read");
+		if (hs[5] != 0.0 || !(std::sqrt(hs[2]) > tol)) break;
+		if (it >= d.max_iterations) {
+			if (iterations) *iterations = it;
+			return set_error(IBK_ERR_DEVICE_CHECK, kNoConvergence);
+		}
+		launch_march(d.ops, 2, d.march, dv, q, pa, s);
+		alpha_kernel<<<1, kSumThreads, 0, s>>>(pa, d.march.blocks(), tol * tol, sc);
+		update_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, sc, dv, q, x, r, diag, pa);
+		beta_kernel<<<1, kSumThreads, 0, s>>>(pa, kFluidBlocks, sc);
+		direction_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, sc, q, dv, pb);
+		sum_kernel<<<1, kSumThreads, 0, s>>>(pb, kFluidBlocks, sc + 2);
+		if ((st = check_launch("diffusion iteration kernels")) != IBK_OK) return st;
+		++it;
+	}
+	// a bail-out leaves the last iteration's update undone, as pcg.h does
+	if (hs[5] != 0.0 && it > 0) --it;
+	finish_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, u, x, out);
+	if (iterations) *iterations = it;
+	return check_launch("finish_kernel");
+}
+
+} // namespace
 
 extern "C" {
 
@@ -556,20 +1138,44 @@ ibk_status ibk_diffusion_create(ibk_plan plan, int component, const double robin
 		d->ops.ax[a].periodic = periodic;
 		off += 4 * P;
 	}
-	d->march_grid = dim3((unsigned) ((d->ops.ax[0].P + kMarchX - 1) / kMarchX),
-	                     (unsigned) ((d->ops.ax[1].P + kMarchY - 1) / kMarchY),
-	                     (unsigned) ((d->ops.ax[2].P + kMarchZ - 1) / kMarchZ));
-	d->march_blocks = (int) (d->march_grid.x * d->march_grid.y * d->march_grid.z);
-	if (d->march_grid.y > 65535u || d->march_grid.z > 65535u || size >= (1LL << 31)) {
-		delete d;
-		return set_error(IBK_ERR_UNSUPPORTED, "grid too large for the operator kernel (2^31 faces)");
-	}
-	const int first_partials = std::max(d->march_blocks, kFluidBlocks);
+	const int P0 = d->ops.ax[0].P, P1 = d->ops.ax[1].P, P2 = d->ops.ax[2].P;
+	const auto tiles = [](int p, int t) { return (unsigned) ((p + t - 1) / t); };
+	d->march.grid = dim3(tiles(P0, kMarchX), tiles(P1, kMarchY), 1);
+	while (d->march.zrun > 2 && (long long) d->march.grid.x * d->march.grid.y * tiles(P2, d->march.zrun) < 4LL * p->num_sms)
+		d->march.zrun /= 2;
+	d->march.grid.z = tiles(P2, d->march.zrun);
+	d->dir_grid = dim3(tiles(P0, kDirX), tiles(P1, kDirY), 1);
+	d->dir_run = pick_run((long long) d->dir_grid.x * d->dir_grid.y, P2, 1, (long long) kDirBlocks * p->num_sms).planes;
+	d->dir_grid.z = tiles(P2, d->dir_run);
+	// the wide tile's step takes kWideStep times as long as the small one's
+	const dim3 wide(tiles(P0, PolyWide::X), tiles(P1, PolyWide::Y), 1), small(tiles(P0, PolySmall::X), tiles(P1, PolySmall::Y), 1);
+	const Run rw = pick_run((long long) wide.x * wide.y, P2, PolyWide::HALO, (long long) PolyWide::BLOCKS * p->num_sms);
+	const Run rs = pick_run((long long) small.x * small.y, P2, PolySmall::HALO, (long long) PolySmall::BLOCKS * p->num_sms);
+	d->poly_wide = kWideStep * rw.cost <= rs.cost;
+	d->poly_grid = d->poly_wide ? wide : small;
+	d->poly_run = (d->poly_wide ? rw : rs).planes;
+	d->poly_grid.z = tiles(P2, d->poly_run);
+	for (const dim3& g : {d->march.grid, d->dir_grid, d->poly_grid})
+		if (g.y > 65535u || g.z > 65535u || size >= (1LL << 31)) {
+			delete d;
+			return set_error(IBK_ERR_UNSUPPORTED, "grid too large for the operator kernel (2^31 faces)");
+		}
+	const auto count = [](const dim3& g) { return (int) (g.x * g.y * g.z); };
+	d->first_partials = std::max({count(d->march.grid), 2 * count(d->dir_grid), count(d->poly_grid), kFluidBlocks});
 	cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d->coef), sizeof(double) * (size_t) total);
 	if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->work), sizeof(double) * 8 * (size_t) size);
 	if (e == cudaSuccess)
-		e = cudaMalloc(reinterpret_cast<void**>(&d->partial), sizeof(double) * (size_t) (first_partials + kFluidBlocks));
-	if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->scalars), sizeof(double) * 8);
+		e = cudaMalloc(reinterpret_cast<void**>(&d->partial), sizeof(double) * (size_t) (d->first_partials + kFluidBlocks));
+	if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d->scalars), sizeof(double) * (kScalars + 1));
+	if (e == cudaSuccess)
+		e = cudaHostAlloc(reinterpret_cast<void**>(&d->host_tests), sizeof(double) * 2 * (kLookAhead + 1),
+		                  cudaHostAllocMapped);
+	for (cudaEvent_t& ev : d->tested)
+		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(polynomial_kernel<PolyWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, PolyWide::BYTES);
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(polynomial_kernel<PolySmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, PolySmall::BYTES);
 	if (e == cudaSuccess) e = cudaMemcpy(d->coef, host.data(), sizeof(double) * (size_t) total, cudaMemcpyHostToDevice);
 	if (e != cudaSuccess) {
 		cudaGetLastError();
@@ -643,6 +1249,9 @@ ibk_status ibk_diffusion_destroy(ibk_diffusion d)
 	cudaFree(d->work);
 	cudaFree(d->partial);
 	cudaFree(d->scalars);
+	for (cudaEvent_t ev : d->tested)
+		if (ev) cudaEventDestroy(ev);
+	if (d->host_tests) cudaFreeHost(d->host_tests);
 	cudaSetDevice(dev);
 	delete d;
 	return IBK_OK;
@@ -652,7 +1261,7 @@ ibk_status ibk_diffusion_apply(ibk_diffusion d, int op, const double* u, double*
 {
 	if (!d || !u || !out || op < 0 || op > 2) return set_error(IBK_ERR_INVALID_ARGUMENT, "null arrays or unknown operator");
 	cudaStream_t s = static_cast<cudaStream_t>(stream);
-	launch_march(d->ops, op, d->march_grid, u, out, nullptr, s);
+	launch_march(d->ops, op, d->march, u, out, nullptr, s);
 	return check_launch("march_apply_kernel");
 }
 
@@ -660,88 +1269,8 @@ ibk_status ibk_diffusion_step(ibk_diffusion d, double gamma, const double* u, co
                               double* out, int* iterations, void* stream)
 {
 	if (!d || !u || !rhs || !f || !out) return set_error(IBK_ERR_INVALID_ARGUMENT, "null arrays");
-	cudaStream_t s = static_cast<cudaStream_t>(stream);
-	const long long n = d->ops.size;
-	double* b = d->work;
-	double* r = b + n;
-	double* dv = r + n;
-	double* q = dv + n;
-	double* x = q + n;
-	double* diag = x + n;
-	double* tmp = diag + n;
-	double* tmp2 = tmp + n;
-	double* pa = d->partial;                                            // march_blocks or kFluidBlocks
-	double* pb = d->partial + std::max(d->march_blocks, kFluidBlocks);   // kFluidBlocks
-	double* sc = d->scalars;
-	const double k = gamma * d->timestep;
-	const bool cheb = d->precond == IBK_PRECOND_CHEBYSHEV;
-	const double* w = d->cheb_w;
-	// rhs of the solve: k I~ f + k mu (L u + rhs)
-	const dim3 mg = d->march_grid;
-	launch_march(d->ops, 0, mg, u, tmp, nullptr, s);
-	launch_march(d->ops, 1, mg, f, q, nullptr, s);
-	rhs_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, k, k * d->mu, tmp, rhs, q, b);
-	cudaError_t e = cudaMemcpyAsync(r, b, sizeof(double) * (size_t) n, cudaMemcpyDeviceToDevice, s);
-	if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync");
-	// z = M^-1 r with the r . z partials in pa: the Chebyshev polynomial
-	// (algo/chebyshev.h:152-167: s = w0 r, then s = w_i r - H s, i = 1..3)
-	auto chebyshev = [&](double* z) {
-		launch_march(d->ops, 4, mg, r, tmp, nullptr, s, r, w[1], w[0]);
-		launch_march(d->ops, 3, mg, tmp, tmp2, nullptr, s, r, w[2]);
-		launch_march(d->ops, 3, mg, tmp2, z, pa, s, r, w[3]);
-	};
-	int za = kFluidBlocks;       // the count of r . z partials
-	if (cheb) {
-		// pcg.h:14-18: x = 0, d = M^-1 r, delta = r . d
-		e = cudaMemsetAsync(x, 0, sizeof(double) * (size_t) n, s);
-		if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
-		chebyshev(dv);
-		norm_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, dv, pb);
-		za = d->march_blocks;
-	} else {
-		start_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, r, diag, x, dv, pa, pb);
-	}
-	sum_kernel<<<1, kSumThreads, 0, s>>>(pa, za, sc + 0);
-	sum_kernel<<<1, kSumThreads, 0, s>>>(pb, kFluidBlocks, sc + 2);
-	ibk_status st = check_launch("diffusion set-up kernels");
-	if (st != IBK_OK) return st;
-	e = cudaMemsetAsync(sc + 5, 0, sizeof(double), s);
-	if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
-	const double tol = d->tolerance;
-	int it = 0;
-	double hs[6];
-	for (;;) {
-		// the loop test of pcg.h:21 (|d| > tol) and its bail-out, read back once
-		// per iteration; alpha and beta stay on the device
-		e = cudaMemcpyAsync(hs, sc, sizeof(double) * 6, cudaMemcpyDeviceToHost, s);
-		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-		if (e != cudaSuccess) return cuda_fail(e, "diffusion residual read");
-		if (hs[5] != 0.0 || !(std::sqrt(hs[2]) > tol)) break;
-		if (it >= d->max_iterations) {
-			if (iterations) *iterations = it;
-			return set_error(IBK_ERR_DEVICE_CHECK, "diffusion solve did not converge within max_iterations");
-		}
-		launch_march(d->ops, 2, mg, dv, q, pa, s);
-		alpha_kernel<<<1, kSumThreads, 0, s>>>(pa, d->march_blocks, tol * tol, sc);
-		if (cheb) {
-			// x += alpha d, r -= alpha q, q = M^-1 r (a bail-out leaves x and r as
-			// they are; the polynomial of the unchanged r is then not used)
-			update_xr_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, sc, dv, q, x, r);
-			chebyshev(q);
-		} else {
-			update_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, sc, dv, q, x, r, diag, pa);
-		}
-		beta_kernel<<<1, kSumThreads, 0, s>>>(pa, za, sc);
-		direction_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, sc, q, dv, pb);
-		sum_kernel<<<1, kSumThreads, 0, s>>>(pb, kFluidBlocks, sc + 2);
-		if ((st = check_launch("diffusion iteration kernels")) != IBK_OK) return st;
-		++it;
-	}
-	// a bail-out leaves the last iteration's update undone, as pcg.h does
-	if (hs[5] != 0.0 && it > 0) --it;
-	finish_kernel<<<kFluidBlocks, kFluidThreads, 0, s>>>(n, u, x, out);
-	if (iterations) *iterations = it;
-	return check_launch("finish_kernel");
+	return d->precond == IBK_PRECOND_CHEBYSHEV ? step_chebyshev(*d, gamma, u, rhs, f, out, iterations, static_cast<cudaStream_t>(stream))
+	                                           : step_jacobi(*d, gamma, u, rhs, f, out, iterations, static_cast<cudaStream_t>(stream));
 }
 
 } // extern "C"
