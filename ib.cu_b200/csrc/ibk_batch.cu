@@ -203,10 +203,9 @@ __device__ __forceinline__ void next_item(int* next, int nitems, int nact, const
 	*local = k - __ldg(pre + j);
 }
 
-// Persistent spread over the active instances' items: tiles (FP32C, every
-// component) or (tile, component) (FP64).
-template <typename D, int DIMS, int PREC, int NT = kTileThreads>
-__global__ void __launch_bounds__(NT, PREC == IBK_PRECISION_FP32C ? 1024 / NT : 3)
+// Persistent FP32C spread over the active instances' tiles (every component).
+template <typename D, int DIMS, int NT = kTileThreads>
+__global__ void __launch_bounds__(NT, 1024 / NT)
 batch_spread_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __restrict__ next,
                     const PointRec* __restrict__ recs, const int* __restrict__ off, const unsigned* __restrict__ binmax,
                     int step, Deferral defer)
@@ -224,15 +223,35 @@ batch_spread_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __re
 		copy_to_shared(&so, t.io + inst);
 		__syncthreads();
 		const CompPtrs& fe = so.fe;
-		if constexpr (PREC == IBK_PRECISION_FP32C) {
-			const BinStatsView bs{binmax + (size_t) si.bin_s * kMaxDims};
-			// a dense tile is deferred by its work-item index
-			spread_tile<D, DIMS, PREC, false, NT>(si.g, si.ts, so.n, step ? so.xn : so.x, step ? so.fs : so.fl, recs,
-			                                      so.pbase, off + si.bin_s, bs, fe, local, -1, defer, item);
-		} else {
-			spread_tile<D, DIMS, PREC>(si.g, si.ts, so.n, step ? so.xn : so.x, step ? so.fs : so.fl, recs, so.pbase,
-			                           off + si.bin_s, BinStatsView{nullptr}, fe, local / DIMS, local % DIMS);
-		}
+		const BinStatsView bs{binmax + (size_t) si.bin_s * kMaxDims};
+		// a dense tile is deferred by its work-item index
+		spread_tile<D, DIMS, false, NT>(si.g, si.ts, so.n, step ? so.fs : so.fl, recs, so.pbase, off + si.bin_s, bs, fe,
+		                                local, -1, defer, item);
+		__syncthreads();
+	}
+}
+
+// Persistent FP64 spread over the active instances' (tile, component) items.
+template <typename D, int DIMS>
+__global__ void __launch_bounds__(s64_threads<DIMS>(), 4)
+batch_spread64_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __restrict__ next,
+                      const PointRec* __restrict__ recs, const int* __restrict__ off, int step)
+{
+	__shared__ int cur_inst, cur_local;
+	__shared__ BatchInst si;
+	__shared__ BatchIO so;
+	const int nitems = __ldg(&t.hdr->items_s), nact = __ldg(&t.hdr->num_active);
+	for (;;) {
+		if (threadIdx.x == 0) next_item(next, nitems, nact, t.spre, t.active, &cur_inst, &cur_local);
+		__syncthreads();
+		const int inst = cur_inst, local = cur_local;
+		if (inst < 0) return;
+		copy_to_shared(&si, insts + inst);
+		copy_to_shared(&so, t.io + inst);
+		__syncthreads();
+		const CompPtrs& fe = so.fe;
+		spread_any64<D, DIMS>(si.g, si.ts, so.n, step ? so.xn : so.x, step ? so.fs : so.fl, recs, so.pbase,
+		                      off + si.bin_s, fe, local / DIMS, local % DIMS);
 		__syncthreads();
 	}
 }
@@ -265,8 +284,8 @@ batch_spread_dense_kernel(const BatchInst* __restrict__ insts, BatchTable t, con
 		__syncthreads();
 		const CompPtrs& fe = so.fe;
 		const BinStatsView bs{binmax + (size_t) si.bin_s * kMaxDims};
-		spread_tile<D, DIMS, IBK_PRECISION_FP32C, true>(si.g, si.ts, so.n, step ? so.xn : so.x, step ? so.fs : so.fl,
-		                                                recs, so.pbase, off + si.bin_s, bs, fe, cur_local, cur_comp);
+		spread_tile<D, DIMS, true>(si.g, si.ts, so.n, step ? so.fs : so.fl, recs, so.pbase, off + si.bin_s, bs, fe,
+		                           cur_local, cur_comp);
 		__syncthreads();
 	}
 }
@@ -444,19 +463,20 @@ ibk_status batch_run_impl(Batch& b, int op, cudaStream_t s)
 		return check_launch("batch_interp_kernel");
 	};
 	auto spread = [&]() -> ibk_status {
-		Deferral defer{b.d_defer + 4, b.d_defer};
-		if (PREC == IBK_PRECISION_FP32C) {
+		b.launches += 1;
+		if constexpr (PREC == IBK_PRECISION_FP64) {
+			batch_spread64_kernel<D, DIMS><<<b.grid_s, s64_threads<DIMS>(), b.smem_s, s>>>(
+				b.d_inst, t, b.d_next, b.d_recs, b.d_off, step ? 1 : 0);
+		} else {
+			Deferral defer{b.d_defer + 4, b.d_defer};
 			ibk_status ds = cuda_check(cudaMemsetAsync(b.d_defer, 0, sizeof(int), s), "cudaMemsetAsync");
 			if (ds != IBK_OK) return ds;
-		}
-		if (PREC == IBK_PRECISION_FP32C && b.config.spread_threads == 512)
-			batch_spread_kernel<D, DIMS, PREC, 512><<<b.grid_s, 512, b.smem_s, s>>>(
-				b.d_inst, t, b.d_next, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer);
-		else
-			batch_spread_kernel<D, DIMS, PREC><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
-				b.d_inst, t, b.d_next, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer);
-		b.launches += 1;
-		if (PREC == IBK_PRECISION_FP32C) {
+			if (b.config.spread_threads == 512)
+				batch_spread_kernel<D, DIMS, 512><<<b.grid_s, 512, b.smem_s, s>>>(
+					b.d_inst, t, b.d_next, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer);
+			else
+				batch_spread_kernel<D, DIMS><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
+					b.d_inst, t, b.d_next, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer);
 			batch_spread_dense_kernel<D, DIMS><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
 				b.d_inst, t, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer.list, defer.count);
 			b.launches += 1;
@@ -486,23 +506,29 @@ template <int KIND, int ORDER, int DIMS, int PREC>
 ibk_status batch_prepare_impl(Batch& b)
 {
 	using D = Delta<KIND, ORDER>;
-	const bool wide = PREC == IBK_PRECISION_FP32C && b.config.spread_threads == 512;
-	auto ks = wide ? batch_spread_kernel<D, DIMS, PREC, 512> : batch_spread_kernel<D, DIMS, PREC>;
-	const int nts = wide ? 512 : kTileThreads;
 	auto ki = batch_interp_kernel<D, DIMS, PREC>;
 	ibk_status st;
+	int occ_s = 0, occ_i = 0;
+	// the spread kernel's shared memory and resident CTAs
+	auto prepare_spread = [&](auto ks, int nts) -> ibk_status {
+		ibk_status ps = cuda_check(cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_s),
+		                           "cudaFuncSetAttribute");
+		if (ps != IBK_OK) return ps;
+		return cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks, nts, b.smem_s),
+		                  "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+	};
 	if constexpr (PREC == IBK_PRECISION_FP32C) {
 		if ((st = cuda_check(cudaFuncSetAttribute(batch_spread_dense_kernel<D, DIMS>,
 		                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_s),
 		                     "cudaFuncSetAttribute")) != IBK_OK) return st;
+		st = b.config.spread_threads == 512 ? prepare_spread(batch_spread_kernel<D, DIMS, 512>, 512)
+		                                    : prepare_spread(batch_spread_kernel<D, DIMS>, kTileThreads);
+	} else {
+		st = prepare_spread(batch_spread64_kernel<D, DIMS>, s64_threads<DIMS>());
 	}
-	if ((st = cuda_check(cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_s),
-	                     "cudaFuncSetAttribute")) != IBK_OK) return st;
+	if (st != IBK_OK) return st;
 	if ((st = cuda_check(cudaFuncSetAttribute(ki, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_i),
 	                     "cudaFuncSetAttribute")) != IBK_OK) return st;
-	int occ_s = 0, occ_i = 0;
-	if ((st = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks, nts, b.smem_s),
-	                     "cudaOccupancyMaxActiveBlocksPerMultiprocessor")) != IBK_OK) return st;
 	if ((st = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_i, ki, kTileThreads, b.smem_i),
 	                     "cudaOccupancyMaxActiveBlocksPerMultiprocessor")) != IBK_OK) return st;
 	if (occ_s < 1 || occ_i < 1) return set_error(IBK_ERR_UNSUPPORTED, "batch tiles need more shared memory than an SM has");
@@ -624,7 +650,7 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 	std::vector<BatchInst> inst(b.count);
 	std::vector<int> nitem_s(b.count), nitem_i(b.count);
 	long long bins_s = 0, bins_i = 0, items_s = 0, items_i = 0;
-	size_t smem_max = 0, region_max = 0;
+	size_t smem_max = 0, limit_max = 0, region_max = 0;
 	for (int i = 0; i < b.count; ++i) {
 		BatchInst& bi = inst[i];
 		bi.g = b.geo[i];
@@ -651,10 +677,11 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 		if (bins_s >= (1LL << 30) || bins_i >= (1LL << 30) || items_s >= (1LL << 30) || items_i >= (1LL << 30))
 			return set_error(IBK_ERR_INVALID_ARGUMENT, "batch has too many tiles");
 		smem_max = std::max(smem_max, spread_tile_bytes(bi.g, bi.ts, b.M, b.precision));
+		limit_max = std::max(limit_max, spread_limit_bytes(bi.g, bi.ts, b.M, b.precision));
 		region_max = std::max(region_max, interp_region_bytes(bi.g, bi.ti, b.M));
 	}
 	const size_t smem_s = smem_max;
-	if (smem_s > 200 * 1024 || region_max > 200 * 1024)
+	if (limit_max > 200 * 1024 || region_max > 200 * 1024)
 		return set_error(IBK_ERR_UNSUPPORTED, "batch tile shape needs more than 200 KB of shared memory");
 	ibk_status st;
 	const size_t nb = (size_t) std::max(bins_s, bins_i);

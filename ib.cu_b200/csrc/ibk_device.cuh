@@ -194,6 +194,70 @@ template <int ORDER> struct Delta<kHat, ORDER> {
 	static __device__ __forceinline__ float phi32(float r) { return 1.0f - fabsf(r); }
 };
 
+// All M weights of one axis in FP64 for fractional offset delta, bit-exact
+// with phi64 (= the reference) at delta + (m - (M - 1) / 2).
+template <typename D>
+__device__ __forceinline__ void weights64(double delta, double* w)
+{
+	constexpr int sh = (D::M - 1) >> 1;
+#pragma unroll
+	for (int m = 0; m < D::M; ++m) w[m] = D::phi64(__dadd_rn(delta, (double) (m - sh)));
+}
+
+// r / 3, correctly rounded: Markstein's theorem (a quotient within one unit
+// in the last place, corrected once by its exact remainder times the rounded
+// reciprocal).
+__device__ __forceinline__ double third(double r)
+{
+	constexpr double y = 1.0 / 3.0;
+	const double q = __dmul_rn(r, y);
+	return __fma_rn(__fma_rn(-3.0, q, r), y, q);
+}
+
+static __device__ __noinline__ double bspline3_recursion(double r) { return BsplineFn<3>::eval64(r); }
+
+// bspline<3>: each weight's interval is known from m, so of the recursion's
+// eight indicator functions only those that are 1 are written out (a
+// product with 0 or 1 and a sum with 0 are exact); 19 FP64 operations a
+// weight instead of about 60.  Closer to 0 than 2^-50 the recursion's own
+// roundings of delta +- 1/2 let both neighbouring indicators (or neither) be
+// 1, so there it is evaluated as it stands; 0 itself is regular.
+template <>
+__device__ __forceinline__ void weights64<Delta<kBspline, 3>>(double delta, double* w)
+{
+	if (!(delta <= -0x1p-50 || delta == 0.0)) {
+		w[0] = bspline3_recursion(__dadd_rn(delta, -1.0));
+		w[1] = bspline3_recursion(__dadd_rn(delta, 0.0));
+		w[2] = bspline3_recursion(__dadd_rn(delta, 1.0));
+		w[3] = bspline3_recursion(__dadd_rn(delta, 2.0));
+		return;
+	}
+	constexpr double b = 4.0 / 6.0;
+	// bspline<2> on its outer intervals and bspline<1>, as products (c + s / 2)(1 +- t)
+	auto up = [](double s, double t) { return __dmul_rn(__dadd_rn(0.75, __dmul_rn(s, 0.5)), t); };
+	auto down = [](double s, double t) { return __dmul_rn(__dsub_rn(0.75, __dmul_rn(s, 0.5)), t); };
+	{
+		const double r = __dadd_rn(delta, -1.0), s = __dadd_rn(r, 0.5);
+		w[0] = __dmul_rn(__dadd_rn(b, third(r)), up(s, __dadd_rn(1.0, __dadd_rn(s, 0.5))));
+	}
+	{
+		const double r = __dadd_rn(delta, 0.0), a = third(r), s = __dadd_rn(r, 0.5), h = __dsub_rn(r, 0.5);
+		const double lo = __dadd_rn(up(s, __dsub_rn(1.0, __dadd_rn(s, 0.5))), down(s, __dadd_rn(1.0, __dsub_rn(s, 0.5))));
+		const double hi = up(h, __dadd_rn(1.0, __dadd_rn(h, 0.5)));
+		w[1] = __dadd_rn(__dmul_rn(__dadd_rn(b, a), lo), __dmul_rn(__dsub_rn(b, a), hi));
+	}
+	{
+		const double r = __dadd_rn(delta, 1.0), a = third(r), s = __dadd_rn(r, 0.5), h = __dsub_rn(r, 0.5);
+		const double lo = down(s, __dsub_rn(1.0, __dsub_rn(s, 0.5)));
+		const double hi = __dadd_rn(up(h, __dsub_rn(1.0, __dadd_rn(h, 0.5))), down(h, __dadd_rn(1.0, __dsub_rn(h, 0.5))));
+		w[2] = __dadd_rn(__dmul_rn(__dadd_rn(b, a), lo), __dmul_rn(__dsub_rn(b, a), hi));
+	}
+	{
+		const double r = __dadd_rn(delta, 2.0), s = __dsub_rn(r, 0.5);
+		w[3] = __dmul_rn(__dsub_rn(b, third(r)), down(s, __dsub_rn(1.0, __dsub_rn(s, 0.5))));
+	}
+}
+
 // ---------------------------------------------------------- patterns ---
 // standard_pattern / every_other_pattern (include/ib/delta.h:97-147): entry
 // e of the stencil -> offset index m (0..M-1) along dimension j, where the

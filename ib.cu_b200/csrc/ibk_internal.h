@@ -88,9 +88,11 @@ enum { kSlotCount = 0, kSlotOffset = 1, kSlotKeyRank = 2, kSlotRecs = 3, kSlotCh
 // origins in 8 bits).
 constexpr int kMaxTileExtent = 64;
 
-// Shared memory of a spread CTA for tiles tg, and of an interpolation CTA's
-// staged region (largest component, stencil width M), in bytes.
+// Shared memory of a spread CTA for tiles tg, what of it counts against the
+// limit on tile shapes, and an interpolation CTA's staged region (largest
+// component, stencil width M), in bytes.
 size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision);
+size_t spread_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision);
 size_t interp_region_bytes(const GridGeom& g, const TileGeom& tg, int M);
 // Staged interpolation region of component c relative to a tile's first
 // cell: lower corner and extent per axis (the TMA box).

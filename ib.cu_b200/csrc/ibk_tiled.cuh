@@ -12,8 +12,8 @@
 //            products, each rounded once to a per-(tile, component) fixed
 //            point and summed exactly with 32-bit integer shared atomics
 //            (order-independent; see the fixed-point notes below).
-//     FP64:  one CTA per (tile, component), FP64 shared-memory accumulation,
-//            the reference's exact weights.
+//     FP64:  one CTA per (tile, component), the reference's exact weights,
+//            FP64 sums in shared memory that one warp owns (spread_tile64).
 //
 // interp_tile  -- one CTA per (tile, component) stages the tile plus the
 //   stencil halo of that component in shared memory with one TMA bulk tensor
@@ -27,6 +27,7 @@
 //            sums of M products, FP64 sum of the rows.
 #pragma once
 #include <algorithm>
+#include <type_traits>
 #include "ibk_device.cuh"
 #include "ibk_bin.cuh"
 #include "ibk_tma.cuh"
@@ -217,10 +218,6 @@ __device__ __forceinline__ int range_walk(const RangeTable& rt, int& r, int item
 }
 
 // ------------------------------------------------------------ spread ---
-
-template <int PREC> struct SpreadAcc;
-template <> struct SpreadAcc<IBK_PRECISION_FP64> { using type = double; };
-template <> struct SpreadAcc<IBK_PRECISION_FP32C> { using type = int; };
 
 // Fixed point of the FP32C spread.  Per (tile, component) a power-of-two
 // scale is chosen so that every single |term| stays below 2^22, the largest
@@ -496,8 +493,7 @@ __device__ __forceinline__ int local_node(int j, int e, int cells, bool wrap, bo
 	return j;
 }
 
-// The general form of spread_fix / spread_f64 for tiles with a wrapping
-// axis: per-node local indices (each face of the tile may be reached from
+// The general form of spread_fix for tiles with a wrapping axis: per-node local indices (each face of the tile may be reached from
 // both sides of the period).
 template <typename D, int DIMS, typename Acc, typename Term>
 __device__ __forceinline__ void spread_wrapped(const int* l, const int* e, const int* cells, const bool* wrap,
@@ -526,44 +522,6 @@ __device__ __forceinline__ void spread_wrapped(const int* l, const int* e, const
 #pragma unroll
 		for (int m0 = 0; m0 < M; ++m0)
 			if ((mk[0] >> m0) & 1u) add(row + loc[0][m0], weight_row(m0, m1, m2));
-	}
-}
-
-// FP64 contribution set (the reference's arithmetic: w0 * (res F) times
-// w1 * w2, exact weights), tile without wrapping axes.
-template <typename D, int DIMS>
-__device__ __forceinline__ void spread_f64(double* acc, const int* l, const double* dl, double f, const int* e,
-                                           int S1, int S2)
-{
-	constexpr int M = D::M, sh = (M - 1) >> 1;
-	unsigned mk[DIMS];
-	bool any = true;
-#pragma unroll
-	for (int d = 0; d < DIMS; ++d) {
-		mk[d] = axis_mask<M>(l[d] - sh, e[d]);
-		any = any && mk[d] != 0u;
-	}
-	if (!any) return;
-	double w[DIMS][M];
-#pragma unroll
-	for (int d = 0; d < DIMS; ++d)
-#pragma unroll
-		for (int m = 0; m < M; ++m)
-			w[d][m] = (mk[d] >> m & 1u) ? D::phi64(__dadd_rn(dl[d], (double) (m - sh))) : 0.0;
-#pragma unroll
-	for (int m0 = 0; m0 < M; ++m0) w[0][m0] = __dmul_rn(w[0][m0], f);
-	const int first = (l[0] - sh) + (l[1] - sh) * S1 + (DIMS == 3 ? (l[2] - sh) * S2 : 0);
-	constexpr int R = DIMS == 3 ? M * M : M;
-#pragma unroll
-	for (int r = 0; r < R; ++r) {
-		const int m1 = r % M, m2 = r / M;
-		const unsigned rm = DIMS == 3 ? (mk[1] >> m1) & (mk[2] >> m2) & 1u : (mk[1] >> m1) & 1u;
-		if (!rm) continue;
-		const double w12 = DIMS == 3 ? __dmul_rn(w[1][m1], w[2][m2]) : w[1][m1];
-		double* row = acc + first + m1 * S1 + (DIMS == 3 ? m2 * S2 : 0);
-#pragma unroll
-		for (int m0 = 0; m0 < M; ++m0)
-			if ((mk[0] >> m0) & 1u) atomicAdd(row + m0, __dmul_rn(w[0][m0], w12));
 	}
 }
 
@@ -662,12 +620,12 @@ __device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const Tile
 	}
 }
 
-// One spread tile; every thread of the CTA calls it.  comp < 0: every
-// component (FP32C); else that component only (FP64).  Records carry point
-// indices offset by pbase (a batch numbers the points of all its instances
-// consecutively); off is this grid's bin table.
-// Dense tiles (FP32C tiles where a face may receive more terms than a
-// 32-bit word holds) are not summed by the one-pass kernel: it appends
+// One FP32C spread tile; every thread of the CTA calls it.  FOLDED takes one
+// component comp of a deferred tile, else every component.  Records carry
+// point indices offset by pbase (a batch numbers the points of all its
+// instances consecutively); off is this grid's bin table.
+// Dense tiles (tiles where a face may receive more terms than a 32-bit word
+// holds) are not summed by the one-pass kernel: it appends
 // (defer_id << 2) | c for each component c to the deferral list and leaves
 // the tile to the folded kernel, one component per item, which keeps the
 // folded form out of the one-pass kernel's code.
@@ -676,14 +634,13 @@ struct Deferral {
 	int* count;
 };
 
-template <typename D, int DIMS, int PREC, bool FOLDED = false, int NT = kTileThreads>
-__device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& tg, int n, const double* __restrict__ x,
+template <typename D, int DIMS, bool FOLDED = false, int NT = kTileThreads>
+__device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& tg, int n,
                                             const double* __restrict__ fl, const PointRec* __restrict__ recs, int pbase,
                                             const int* __restrict__ off, BinStatsView bs, const CompPtrs& fe,
                                             int tile, int comp, Deferral defer = Deferral{nullptr, nullptr},
                                             int defer_id = 0)
 {
-	using acc_t = typename SpreadAcc<PREC>::type;
 	constexpr int M = D::M;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ RangeTable rt;
@@ -691,8 +648,8 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 
 	const int T0 = tg.T[0], T1 = tg.T[1], T2 = DIMS == 3 ? tg.T[2] : 1;
 	const SpreadStrides ss = spread_strides(T0, T1, T2, DIMS);
-	const int c_lo = comp < 0 ? 0 : comp, c_hi = comp < 0 ? DIMS : comp + 1;
-	acc_t* acc = reinterpret_cast<acc_t*>(smem_raw + 4 * kGuardWords);
+	const int c_lo = FOLDED ? comp : 0, c_hi = FOLDED ? comp + 1 : DIMS;
+	int* acc = reinterpret_cast<int*>(smem_raw + 4 * kGuardWords);
 	int tc[3] = {0, 0, 0};
 	tile_coords(tg, tile, tc);
 	int lo[3] = {0, 0, 0};
@@ -707,8 +664,7 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 		wrap_any = wrap_any || wrap[d];
 	}
 	__shared__ unsigned s_fmax[kMaxDims];
-	if constexpr (PREC == IBK_PRECISION_FP32C) build_ranges<DIMS>(g, tg, tc, off, rt, bs, s_fmax);
-	else build_ranges<DIMS>(g, tg, tc, off, rt);
+	build_ranges<DIMS>(g, tg, tc, off, rt, bs, s_fmax);
 	const int ncand = rt.pref[rt.count];
 	if (ncand == 0) {
 		// no point reaches the tile: its faces are zero
@@ -721,33 +677,25 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 		return;
 	}
 	const unsigned acc_addr = smem_addr(acc);
-	if constexpr (PREC == IBK_PRECISION_FP32C && FOLDED) {
+	if constexpr (FOLDED) {
 		if (threadIdx.x < kMaxDims) s_scale[threadIdx.x] = fix_scale(s_fmax[threadIdx.x], max_weight<D, DIMS>(), kFoldChunk);
 		spread_tile_folded<D, DIMS, NT>(g, tg, n, fl, recs, pbase, rt, ncand, lo, cells, wrap, wrap_any, acc_addr,
 		                                fe, s_scale, c_lo, c_hi);
 		return;
 	}
-	if constexpr (PREC == IBK_PRECISION_FP32C && !FOLDED) {
-		// one pass unless a face may receive more than 2 kFoldChunk terms (the
-		// occupancy bound uses the accumulator memory before it is zeroed; a
-		// tile that wraps a periodic axis counts every candidate)
-		const int nmax = (ncand <= kFoldChunk || wrap_any)
-			? ncand : window_occupancy<M, DIMS, NT>(g, tg, rt, ncand, recs, reinterpret_cast<int*>(acc));
-		if (nmax > 2 * kFoldChunk) {
-			// one deferred item per component: (defer_id << 2) | component
-			if (threadIdx.x < DIMS) defer.list[atomicAdd(defer.count, 1)] = (defer_id << 2) | (int) threadIdx.x;
-			return;
-		}
-		if (threadIdx.x < kMaxDims) s_scale[threadIdx.x] = fix_scale(s_fmax[threadIdx.x], max_weight<D, DIMS>(), nmax);
+	// one pass unless a face may receive more than 2 kFoldChunk terms (the
+	// occupancy bound uses the accumulator memory before it is zeroed; a
+	// tile that wraps a periodic axis counts every candidate)
+	const int nmax = (ncand <= kFoldChunk || wrap_any)
+		? ncand : window_occupancy<M, DIMS, NT>(g, tg, rt, ncand, recs, acc);
+	if (nmax > 2 * kFoldChunk) {
+		// one deferred item per component: (defer_id << 2) | component
+		if (threadIdx.x < DIMS) defer.list[atomicAdd(defer.count, 1)] = (defer_id << 2) | (int) threadIdx.x;
+		return;
 	}
-	const int nwords = ss.words * (c_hi - c_lo);
-	for (int i = threadIdx.x * 4; i < nwords; i += NT * 4) {
-		if constexpr (PREC == IBK_PRECISION_FP32C) *reinterpret_cast<int4*>(acc + i) = make_int4(0, 0, 0, 0);
-		else {
-			*reinterpret_cast<double2*>(acc + i) = make_double2(0.0, 0.0);
-			*reinterpret_cast<double2*>(acc + i + 2) = make_double2(0.0, 0.0);
-		}
-	}
+	if (threadIdx.x < kMaxDims) s_scale[threadIdx.x] = fix_scale(s_fmax[threadIdx.x], max_weight<D, DIMS>(), nmax);
+	const int nwords = ss.words * DIMS;
+	for (int i = threadIdx.x * 4; i < nwords; i += NT * 4) *reinterpret_cast<int4*>(acc + i) = make_int4(0, 0, 0, 0);
 	__syncthreads();
 
 	int r = 0;
@@ -760,7 +708,7 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 #pragma unroll
 		for (int d = 0; d < DIMS; ++d) lh[d] = rec_origin(rec.org, d) + unpack8(sft, d);
 #pragma unroll 1
-		for (int c = c_lo; c < c_hi; ++c) {
+		for (int c = 0; c < DIMS; ++c) {
 			const CompGeom& cg = g.comp[c];
 			int l[DIMS], e[DIMS];
 #pragma unroll
@@ -769,97 +717,439 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 				l[d] = lh[d] + (own ? rec_own_shift(rec.org, d) : 0);
 				e[d] = min(tg.T[d], cg.points[d] - lo[d]);
 			}
-			if constexpr (PREC == IBK_PRECISION_FP32C) {
-				const float sc = s_scale[c];
-				if (sc == 0.0f) continue;
-				const float f = (float) (g.res * __ldg(fl + (size_t) c * n + p)) * sc;
-				float dl[DIMS];
+			const float sc = s_scale[c];
+			if (sc == 0.0f) continue;
+			const float f = (float) (g.res * __ldg(fl + (size_t) c * n + p)) * sc;
+			float dl[DIMS];
 #pragma unroll
-				for (int d = 0; d < DIMS; ++d) dl[d] = (tg.tag_mac && d == c) ? rec.dn[d] : rec.dh[d];
-				const unsigned a = acc_addr + 4u * (unsigned) (ss.words * (c - c_lo));
-				if (!wrap_any) {
-					spread_fix<D, DIMS>(a, l, dl, f, e, ss.S1, ss.S2);
-				} else {
-					float w[DIMS][M];
-#pragma unroll
-					for (int d = 0; d < DIMS; ++d) weights32<D>(dl[d], w[d]);
-					spread_wrapped<D, DIMS>(l, e, cells, wrap, ss.S1, ss.S2,
-						[&](int li, int v) { red_shared(a + 4u * (unsigned) li, v); },
-						[&](int m0, int m1, int m2) {
-							const float w12 = DIMS == 3 ? w[1][m1] * w[2][m2] : w[1][m1];
-							return fix_term(w[0][m0] * f, w12);
-						});
-				}
+			for (int d = 0; d < DIMS; ++d) dl[d] = (tg.tag_mac && d == c) ? rec.dn[d] : rec.dh[d];
+			const unsigned a = acc_addr + 4u * (unsigned) (ss.words * c);
+			if (!wrap_any) {
+				spread_fix<D, DIMS>(a, l, dl, f, e, ss.S1, ss.S2);
 			} else {
-				const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
-				double dl[DIMS];
+				float w[DIMS][M];
 #pragma unroll
-				for (int d = 0; d < DIMS; ++d) dl[d] = axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta;
-				double* a = reinterpret_cast<double*>(acc) + (size_t) ss.words * (c - c_lo);
-				if (!wrap_any) {
-					spread_f64<D, DIMS>(a, l, dl, f, e, ss.S1, ss.S2);
-				} else {
-					constexpr int sh = (M - 1) >> 1;
-					double w[DIMS][M];
-#pragma unroll
-					for (int d = 0; d < DIMS; ++d)
-#pragma unroll
-						for (int m = 0; m < M; ++m) w[d][m] = D::phi64(__dadd_rn(dl[d], (double) (m - sh)));
-					spread_wrapped<D, DIMS>(l, e, cells, wrap, ss.S1, ss.S2,
-						[&](int li, double v) { atomicAdd(a + li, v); },
-						[&](int m0, int m1, int m2) {
-							const double w12 = DIMS == 3 ? __dmul_rn(w[1][m1], w[2][m2]) : w[1][m1];
-							return __dmul_rn(__dmul_rn(w[0][m0], f), w12);
-						});
-				}
+				for (int d = 0; d < DIMS; ++d) weights32<D>(dl[d], w[d]);
+				spread_wrapped<D, DIMS>(l, e, cells, wrap, ss.S1, ss.S2,
+					[&](int li, int v) { red_shared(a + 4u * (unsigned) li, v); },
+					[&](int m0, int m1, int m2) {
+						const float w12 = DIMS == 3 ? w[1][m1] * w[2][m2] : w[1][m1];
+						return fix_term(w[0][m0] * f, w12);
+					});
 			}
 		}
 	}
 	__syncthreads();
 
 	// every face of the tile, written once
-	for (int c = c_lo; c < c_hi; ++c) {
+	for (int c = 0; c < DIMS; ++c) {
 		int e[3] = {1, 1, 1};
 #pragma unroll
 		for (int d = 0; d < DIMS; ++d) e[d] = min(tg.T[d], g.comp[c].points[d] - lo[d]);
-		const acc_t* ac = acc + (size_t) ss.words * (c - c_lo);
-		if constexpr (PREC == IBK_PRECISION_FP64) {
-			write_tile<DIMS, NT>(fe.p[c], g.comp[c], lo, e, ss.S1, ss.S2, [&](int li) { return ac[li]; });
-		} else {
-			const float sc = s_scale[c];
-			const double inv = sc != 0.0f ? 1.0 / (double) sc : 0.0;
-			write_tile<DIMS, NT>(fe.p[c], g.comp[c], lo, e, ss.S1, ss.S2,
-			                     [&](int li) { return (double) ac[li] * inv; });
+		const int* ac = acc + (size_t) ss.words * c;
+		const float sc = s_scale[c];
+		const double inv = sc != 0.0f ? 1.0 / (double) sc : 0.0;
+		write_tile<DIMS, NT>(fe.p[c], g.comp[c], lo, e, ss.S1, ss.S2, [&](int li) { return (double) ac[li] * inv; });
+	}
+}
+
+// ------------------------------------------------------- spread, FP64 ---
+// One CTA per (tile, component).  Two warps each own half of the tile's planes
+// and add a candidate's contributions to them one candidate at a time, a lane
+// per node, by plain loads and stores: no other warp touches those faces and
+// the nodes of one stencil are distinct, so no atomics are needed.  (A shared
+// FP64 atomic is a compare-and-swap loop: about 2 lanes per clock and SM, 48
+// clocks per candidate and component.)  Two more warps prepare chunks of 32
+// candidates in turn, a thread per candidate: exact FP64 offsets and weights,
+// the force times the x weights, and which nodes each owner takes; a chunk is
+// computed in registers during one chunk of the owners and stored during the
+// next.  256 x 128 x 256 channel, 1.36 M points: 1267 -> 950 us, 31 clocks per
+// candidate and component; the owners' instruction stream bounds it (36
+// instructions a visit at 4 CTAs per SM; half of the issue slots and of the
+// shared-memory pipe are used).  One owner a tile takes 1311 us for the spread
+// and interpolation of that channel against 1297, four owners 1586 (a
+// candidate then has 1.75 visits instead of 1.4).  Rows are padded so that the
+// 4 x 4 (x, y) nodes of half a warp lie in 16 different 64-bit banks.
+constexpr int kS64Owners = 2, kS64Makers = 2, kS64Threads = 128, kS64Chunk = 32;
+
+// Accumulators of an FP64 tile: row stride 4 or 12 (mod 16) while the padded
+// tile stays below 100 KB.
+__host__ __device__ inline SpreadStrides spread64_strides(int T0, int T1, int T2)
+{
+	SpreadStrides st;
+	st.S1 = T0;
+	while ((st.S1 & 7) != 4) ++st.S1;
+	if ((size_t) st.S1 * T1 * T2 * sizeof(double) > 100 * 1024) st.S1 = T0;
+	st.S2 = st.S1 * T1;
+	st.words = (st.S2 * T2 + 1) & ~1;
+	return st;
+}
+
+// Doubles of staged weights per candidate (odd: the preparing threads' stores
+// then spread over the banks).
+template <int M, int DIMS> constexpr int s64_weights() { return (DIMS * M) | 1; }
+
+__host__ __device__ inline size_t spread64_smem_bytes(const GridGeom& g, const TileGeom& tg, int M)
+{
+	if (g.dims == 2) return (size_t) spread_strides(tg.T[0], tg.T[1], 1, 2).words * 8;
+	const size_t words = (size_t) spread64_strides(tg.T[0], tg.T[1], tg.T[2]).words;
+	// two chunks of weights and, per owner, of entries
+	return words * 8 + 2 * kS64Chunk * ((size_t) ((g.dims * M) | 1) * 8 + kS64Owners * sizeof(int2));
+}
+
+// part of parts: this CTA's share of the candidates (parts > 1: sums are added
+// to faces that the caller has zeroed).
+template <typename D, int DIMS>
+__device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom& tg, int n,
+                                              const double* __restrict__ x, const double* __restrict__ fl,
+                                              const PointRec* __restrict__ recs, int pbase,
+                                              const int* __restrict__ off, const CompPtrs& fe, int tile, int c, int part, int parts)
+{
+	constexpr int M = D::M, sh = (M - 1) >> 1, LAST = DIMS - 1;
+	constexpr int W = s64_weights<M, DIMS>();
+	constexpr int NODES = ipow_c(M, DIMS), ROUNDS = (NODES + 31) / 32;
+	constexpr unsigned kAll = (1u << M) - 1u;
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	__shared__ RangeTable rt;
+
+	__shared__ int counts[2][kS64Owners];        // entries per chunk buffer and owner
+
+	const SpreadStrides ss = spread64_strides(tg.T[0], tg.T[1], DIMS == 3 ? tg.T[2] : 1);
+	double* acc = reinterpret_cast<double*>(smem_raw);
+	double* weights = acc + ss.words;
+	int2* entries = reinterpret_cast<int2*>(weights + 2 * kS64Chunk * W);    // [buffer][owner][entry], on 16 bytes
+	const CompGeom& cg = g.comp[c];
+	int tc[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, e[3] = {1, 1, 1};
+	tile_coords(tg, tile, tc);
+	bool wrap_any = false;
+#pragma unroll
+	for (int d = 0; d < DIMS; ++d) {
+		lo[d] = tc[d] * tg.T[d];
+		e[d] = min(tg.T[d], cg.points[d] - lo[d]);
+		wrap_any = wrap_any || (!g.solid[d] && tg.ntiles[d] == 1);
+	}
+	build_ranges<DIMS>(g, tg, tc, off, rt);
+	const int ncand = rt.pref[rt.count];
+	if (ncand == 0) {
+		if (parts == 1) write_tile<DIMS, kS64Threads>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [](int) { return 0.0; });
+		return;
+	}
+	const int all = (ncand + kS64Chunk - 1) / kS64Chunk;
+	const int begin = (int) ((long long) all * part / parts), chunks = (int) ((long long) all * (part + 1) / parts) - begin;
+	if (chunks == 0) return;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const bool owner = warp < kS64Owners;
+	const int maker = warp - kS64Owners;
+	const int quarter = (tg.T[LAST] + kS64Owners - 1) / kS64Owners;     // an owner's faces along the last axis
+
+	// A prepared candidate: its first node (an offset into the tile, or per
+	// axis where a node may wrap), the masks of the nodes that the owners take
+	// (8 bits an axis: of the other axes, and of the last axis per owner; 0:
+	// none) and the weights, x times the force.
+	int base = 0;
+	unsigned both = 0u, last[kS64Owners] = {};
+	double w[DIMS][M];
+	int r = 0;                                   // the range of this thread's previous candidate
+	auto compute = [&](int chunk) {
+		const int it = (begin + chunk) * kS64Chunk + lane;
+#pragma unroll
+		for (int h = 0; h < kS64Owners; ++h) last[h] = 0u;
+		if (it >= ncand) return;
+		const PointRec rec = load_rec(recs + range_walk(rt, r, it));
+		const int sft = rt.shift[r];
+		const int p = rec.p - pbase;
+		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
+		double z[DIMS];
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d) z[d] = __ldg(x + (size_t) d * n + p);
+		bool any = true;
+		base = 0;
+		both = 0u;
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d) {
+			const bool own = tg.tag_mac && d == c;
+			const int j0 = rec_origin(rec.org, d) + unpack8(sft, d) + (own ? rec_own_shift(rec.org, d) : 0) - sh;
+			const bool wrap = !g.solid[d] && tg.ntiles[d] == 1;
+			const unsigned mk = wrap ? kAll : axis_mask<M>(j0, e[d]);
+			any = any && mk != 0u;
+			if (d < LAST) {
+				both |= mk << (8 * d);
+			} else {
+#pragma unroll
+				for (int h = 0; h < kS64Owners; ++h) {
+					if (wrap) {
+						for (int m = 0; m < M; ++m)
+							last[h] |= (unsigned) (wrap_index(j0 + m, tg.cells[d]) / quarter == h) << m;
+					} else {
+						last[h] = mk & axis_mask<M>(j0 - h * quarter, quarter);
+					}
+				}
+			}
+			base += wrap_any ? (j0 + 128) << (8 * d) : j0 * (d == 0 ? 1 : (d == 1 ? ss.S1 : ss.S2));
+		}
+#pragma unroll
+		for (int h = 0; h < kS64Owners; ++h) last[h] = any ? last[h] : 0u;
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d) {
+			weights64<D>(axis_step<M>(g, cg, d, z[d]).delta, w[d]);
+			if (d == 0)
+#pragma unroll
+				for (int m = 0; m < M; ++m) w[0][m] = __dmul_rn(w[0][m], f);
+		}
+	};
+	// ... left for the owners: the weights, and per owner a list of entries
+	// (first node; mask, and the candidate in bits 24 to 28)
+	auto store = [&](int chunk) {
+		const int buf = chunk & 1;
+		double* q = weights + (buf * kS64Chunk + lane) * W;
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d)
+#pragma unroll
+			for (int m = 0; m < M; ++m) q[d * M + m] = w[d][m];
+#pragma unroll
+		for (int h = 0; h < kS64Owners; ++h) {
+			const unsigned list = __ballot_sync(0xffffffffu, last[h] != 0u);
+			if (last[h])
+				entries[(buf * kS64Owners + h) * kS64Chunk + __popc(list & ((1u << lane) - 1u))] =
+					make_int2(base, (int) (both | last[h] << (8 * LAST) | (unsigned) lane << 24));
+			if (lane >= __popc(list)) entries[(buf * kS64Owners + h) * kS64Chunk + lane] = make_int2(0, 0);
+			if (lane == 0) counts[buf][h] = __popc(list);
+		}
+	};
+
+	// this lane's node of each round: its axis indices and its bits of the
+	// entries' masks (a lane without a node has a bit that none holds); a
+	// 4-point stencil's rounds differ in the last index only
+	constexpr bool ALIKE = DIMS == 3 && 32 % (M * M) == 0;
+	int m0[ROUNDS], m1[ROUNDS], m2[ROUNDS];
+	unsigned bits[ROUNDS];
+#pragma unroll
+	for (int q = 0; q < ROUNDS; ++q) {
+		const int v = (ALIKE ? 0 : q * 32) + lane;
+		m0[q] = v % M;
+		m1[q] = (v / M) % M;
+		m2[q] = DIMS == 3 ? v / (M * M) + (ALIKE ? q * (32 / (M * M)) : 0) : 0;
+		const bool none = !ALIKE && v >= NODES;
+		bits[q] = none ? 1u << 31 : 1u << m0[q] | 1u << (8 + m1[q]) | (DIMS == 3 ? 1u << (16 + m2[q]) : 0u);
+		if (none) m0[q] = m1[q] = m2[q] = 0;
+	}
+	auto add = [&](auto wrapped, int chunk) {
+		constexpr bool WRAP = decltype(wrapped)::value;
+		const int buf = chunk & 1, count = counts[buf][warp];
+		const double* wb = weights + buf * kS64Chunk * W;
+		const int2* list = entries + (buf * kS64Owners + warp) * kS64Chunk;
+		if (count == 0) return;
+		// The candidates go two by two: of a pair's work only the load - add -
+		// store of one after the other's is a chain, the rest is for the next
+		// pair and hides behind it.  An odd list ends with an empty entry.
+		double wa[2][ROUNDS], wy[2][ROUNDS], wz[2][ROUNDS];
+		int at[2][ROUNDS];
+		bool on[2][ROUNDS];
+		auto fetch = [&](int4 two) {            // a pair's weights
+#pragma unroll
+			for (int u = 0; u < 2; ++u) {
+				const double* q = wb + ((unsigned) (u ? two.w : two.y) >> 24) * W;
+#pragma unroll
+				for (int i = 0; i < ROUNDS; ++i) {
+					wa[u][i] = ALIKE && i ? wa[u][0] : q[m0[i]];
+					wy[u][i] = ALIKE && i ? wy[u][0] : q[M + m1[i]];
+					wz[u][i] = DIMS == 3 ? q[2 * M + m2[i]] : 1.0;
+				}
+			}
+		};
+		auto locate = [&](int4 two) {           // its nodes
+#pragma unroll
+			for (int u = 0; u < 2; ++u) {
+				const int first = u ? two.z : two.x;
+				const unsigned mask = (unsigned) (u ? two.w : two.y);
+#pragma unroll
+				for (int i = 0; i < ROUNDS; ++i) {
+					on[u][i] = (~mask & bits[i]) == 0u;
+					if constexpr (WRAP) {
+						const int a0 = (first & 255) - 128 + m0[i], a1 = ((first >> 8) & 255) - 128 + m1[i];
+						const int a2 = DIMS == 3 ? ((first >> 16) & 255) - 128 + m2[i] : 0;
+						const bool w0 = !g.solid[0] && tg.ntiles[0] == 1, w1 = !g.solid[1] && tg.ntiles[1] == 1;
+						const bool w2 = DIMS == 3 && !g.solid[2] && tg.ntiles[2] == 1;
+						at[u][i] = (w0 ? wrap_index(a0, tg.cells[0]) : a0) + (w1 ? wrap_index(a1, tg.cells[1]) : a1) * ss.S1 +
+						           (w2 ? wrap_index(a2, tg.cells[2]) : a2) * ss.S2;
+					} else {
+						at[u][i] = first + m0[i] + m1[i] * ss.S1 + m2[i] * ss.S2;
+					}
+				}
+			}
+		};
+		const int4* pairs = reinterpret_cast<const int4*>(list);
+		const int npairs = (count + 1) >> 1;
+		int4 next = pairs[0];
+		fetch(next);
+#pragma unroll 1
+		for (int j = 0; j < npairs; ++j) {
+			locate(next);
+			double v[ROUNDS], t[2][ROUNDS];
+#pragma unroll
+			for (int i = 0; i < ROUNDS; ++i)
+				if (on[0][i]) v[i] = acc[at[0][i]];
+#pragma unroll
+			for (int u = 0; u < 2; ++u)
+#pragma unroll
+				for (int i = 0; i < ROUNDS; ++i)
+					t[u][i] = __dmul_rn(wa[u][i], DIMS == 3 ? __dmul_rn(wy[u][i], wz[u][i]) : wy[u][i]);
+			next = pairs[min(j + 1, npairs - 1)];
+#pragma unroll
+			for (int i = 0; i < ROUNDS; ++i)
+				if (on[0][i]) acc[at[0][i]] = __dadd_rn(v[i], t[0][i]);
+			__syncwarp();           // the next candidate's lanes read what these wrote
+#pragma unroll
+			for (int i = 0; i < ROUNDS; ++i)
+				if (on[1][i]) v[i] = acc[at[1][i]];
+			fetch(next);
+#pragma unroll
+			for (int i = 0; i < ROUNDS; ++i)
+				if (on[1][i]) acc[at[1][i]] = __dadd_rn(v[i], t[1][i]);
+			__syncwarp();
+		}
+	};
+
+	if (owner) {
+		for (int i = threadIdx.x; i < ss.words; i += 32 * kS64Owners) acc[i] = 0.0;
+	} else {
+		if (maker < min(chunks, kS64Makers)) compute(maker);
+		if (maker == 0) store(0);
+	}
+	__syncthreads();
+	for (int k = 0; k < chunks; ++k) {
+		if (owner) {
+			if (wrap_any) add(std::true_type{}, k);
+			else add(std::false_type{}, k);
+		} else if (maker >= kS64Makers) {
+		} else if (maker == ((k + 1) & 1)) {
+			if (k + 1 < chunks) store(k + 1);
+		} else if (k + 2 < chunks) {
+			compute(k + 2);
+		}
+		__syncthreads();
+	}
+	if (parts == 1) {
+		write_tile<DIMS, kS64Threads>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [&](int li) { return acc[li]; });
+	} else {
+		for (int i = threadIdx.x; i < e[0] * e[1] * e[2]; i += kS64Threads) {
+			const int l0 = i % e[0], l1 = i / e[0] % e[1], l2 = i / (e[0] * e[1]);
+			const double v = acc[l2 * ss.S2 + l1 * ss.S1 + l0];
+			if (v != 0.0)
+				atomicAdd(fe.p[c] + ((size_t) (lo[2] + l2) * cg.points[1] + (lo[1] + l1)) * cg.points[0] + lo[0] + l0, v);
 		}
 	}
 }
 
-// Shared memory of a spread CTA: the accumulator words of the components it
-// covers (FP32C: every component, 4 bytes per face, or the occupancy grid if
-// larger; FP64: one component, 8 bytes per face), after the guard words.
+// Two dimensions: one CTA of kTileThreads per (tile, component), a thread per
+// candidate, FP64 shared atomics.  A stencil has at most 36 nodes and a tile
+// few faces, so the owners of spread_tile64 would work through a long chain
+// with half of their lanes idle (24 outlines of 160 points on 240 x 120 cells:
+// 20 us against 30).
+template <typename D>
+__device__ __forceinline__ void spread_tile64_plane(const GridGeom& g, const TileGeom& tg, int n,
+                                                    const double* __restrict__ x, const double* __restrict__ fl,
+                                                    const PointRec* __restrict__ recs, int pbase,
+                                                    const int* __restrict__ off, const CompPtrs& fe, int tile, int c)
+{
+	constexpr int M = D::M, sh = (M - 1) >> 1;
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	__shared__ RangeTable rt;
+	const SpreadStrides ss = spread_strides(tg.T[0], tg.T[1], 1, 2);
+	double* acc = reinterpret_cast<double*>(smem_raw);
+	const CompGeom& cg = g.comp[c];
+	int tc[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, e[3] = {1, 1, 1};
+	bool wrap[2];
+	tile_coords(tg, tile, tc);
+#pragma unroll
+	for (int d = 0; d < 2; ++d) {
+		lo[d] = tc[d] * tg.T[d];
+		e[d] = min(tg.T[d], cg.points[d] - lo[d]);
+		wrap[d] = !g.solid[d] && tg.ntiles[d] == 1;
+	}
+	build_ranges<2>(g, tg, tc, off, rt);
+	const int ncand = rt.pref[rt.count];
+	for (int i = threadIdx.x; i < ss.words; i += kTileThreads) acc[i] = 0.0;
+	__syncthreads();
+	int r = 0;
+	for (int it = threadIdx.x; it < ncand; it += kTileThreads) {
+		const PointRec rec = load_rec(recs + range_walk(rt, r, it));
+		const int sft = rt.shift[r], p = rec.p - pbase;
+		double w[2][M];
+		int at[2][M];
+		unsigned mk[2] = {0u, 0u};
+#pragma unroll
+		for (int d = 0; d < 2; ++d) {
+			const int j0 = rec_origin(rec.org, d) + unpack8(sft, d) + (tg.tag_mac && d == c ? rec_own_shift(rec.org, d) : 0) - sh;
+			weights64<D>(axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta, w[d]);
+#pragma unroll
+			for (int m = 0; m < M; ++m) {
+				bool in;
+				at[d][m] = local_node(j0 + m, e[d], tg.cells[d], wrap[d], in);
+				mk[d] |= (unsigned) in << m;
+			}
+		}
+		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
+#pragma unroll
+		for (int m1 = 0; m1 < M; ++m1)
+#pragma unroll
+			for (int m0 = 0; m0 < M; ++m0)
+				if ((mk[0] >> m0) & (mk[1] >> m1) & 1u)
+					atomicAdd(acc + at[1][m1] * ss.S1 + at[0][m0], __dmul_rn(__dmul_rn(w[0][m0], f), w[1][m1]));
+	}
+	__syncthreads();
+	write_tile<2, kTileThreads>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [&](int li) { return acc[li]; });
+}
+
+// Threads and one tile of the FP64 spread kernels.
+template <int DIMS> constexpr int s64_threads() { return DIMS == 3 ? kS64Threads : kTileThreads; }
+
+template <typename D, int DIMS>
+__device__ __forceinline__ void spread_any64(const GridGeom& g, const TileGeom& tg, int n, const double* __restrict__ x,
+                                             const double* __restrict__ fl, const PointRec* __restrict__ recs, int pbase,
+                                             const int* __restrict__ off, const CompPtrs& fe, int tile, int c, int part = 0,
+                                             int parts = 1)
+{
+	if constexpr (DIMS == 3) spread_tile64<D, 3>(g, tg, n, x, fl, recs, pbase, off, fe, tile, c, part, parts);
+	else spread_tile64_plane<D>(g, tg, n, x, fl, recs, pbase, off, fe, tile, c);
+}
+
+// Shared memory of a spread CTA.  FP32C: every component's accumulator words
+// (4 bytes per face; the folded form's words and totals of one component, or
+// the occupancy grid, where larger) and the guard words.
 __host__ __device__ inline size_t spread_smem_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
 {
-	const int dims = g.dims;
-	const size_t words = (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], dims).words;
-	if (precision != IBK_PRECISION_FP32C) return words * 8 + 4 * kGuardWords;
-	// the region (accumulators, folded words and totals, or the occupancy
-	// grid) and the guard words
+	if (precision != IBK_PRECISION_FP32C) return spread64_smem_bytes(g, tg, M);
+	const size_t words = (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words;
 	const size_t occ = occupancy_words_rt(g, tg, M), acc = words * 3;
 	return ((acc > occ ? acc : occ) + kGuardWords) * 4;
 }
 
-// FP32C: 256-thread CTAs capped at 64 registers so that four fit on an SM
-// (their accumulators take 54 KB each at 16^3 tiles); FP64 ones at 85 so
-// that three fit.
-template <typename D, int DIMS, int PREC>
-__global__ void __launch_bounds__(kTileThreads, PREC == IBK_PRECISION_FP32C ? 4 : 3)
-spread_tile_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
-                   const double* __restrict__ fl, const PointRec* __restrict__ recs,
+// What a tile shape is held to (at most 200 KB; 8 bytes per face of one
+// component in FP64).
+__host__ __device__ inline size_t spread_tile_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
+{
+	if (precision == IBK_PRECISION_FP32C) return spread_smem_bytes(g, tg, M, precision);
+	return (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words * 8 + 4 * kGuardWords;
+}
+
+// 256-thread CTAs capped at 64 registers so that four fit on an SM (their
+// accumulators take 54 KB each at 16^3 tiles).
+template <typename D, int DIMS>
+__global__ void __launch_bounds__(kTileThreads, 4)
+spread_tile_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ fl, const PointRec* __restrict__ recs,
                    const int* __restrict__ off, BinStatsView bs, CompPtrs fe, Deferral defer)
 {
-	// grid: tiles (FP32C) or (tile, component) (FP64)
-	spread_tile<D, DIMS, PREC>(g, tg, n, x, fl, recs, 0, off, bs, fe, blockIdx.x,
-	                           PREC == IBK_PRECISION_FP32C ? -1 : (int) blockIdx.y, defer, blockIdx.x);
+	spread_tile<D, DIMS>(g, tg, n, fl, recs, 0, off, bs, fe, blockIdx.x, -1, defer, blockIdx.x);
+}
+
+// grid: (tile, component, part); four CTAs of 52 KB per SM at 16^3 tiles.
+template <typename D, int DIMS>
+__global__ void __launch_bounds__(s64_threads<DIMS>(), 4)
+spread_tile64_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x, const double* __restrict__ fl,
+                     const PointRec* __restrict__ recs, const int* __restrict__ off, CompPtrs fe)
+{
+	spread_any64<D, DIMS>(g, tg, n, x, fl, recs, 0, off, fe, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
 }
 
 // The deferred dense tiles of an FP32C spread, folded (see Deferral); the
@@ -867,15 +1157,14 @@ spread_tile_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
 // device.
 template <typename D, int DIMS>
 __global__ void __launch_bounds__(kTileThreads, 4)
-spread_dense_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
-                    const double* __restrict__ fl, const PointRec* __restrict__ recs,
+spread_dense_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ fl, const PointRec* __restrict__ recs,
                     const int* __restrict__ off, BinStatsView bs, CompPtrs fe, const int* __restrict__ list,
                     const int* __restrict__ count)
 {
 	const int m = *count;
 	for (int k = blockIdx.x; k < m; k += gridDim.x) {
 		const int v = __ldg(list + k);
-		spread_tile<D, DIMS, IBK_PRECISION_FP32C, true>(g, tg, n, x, fl, recs, 0, off, bs, fe, v >> 2, v & 3);
+		spread_tile<D, DIMS, true>(g, tg, n, fl, recs, 0, off, bs, fe, v >> 2, v & 3);
 		__syncthreads();
 	}
 }
@@ -1199,9 +1488,7 @@ __device__ __forceinline__ bool interp_tile(const GridGeom& g, const TileGeom& t
 			if constexpr (PREC == IBK_PRECISION_FP64) {
 				double w[DIMS][M];
 #pragma unroll
-				for (int d = 0; d < DIMS; ++d)
-#pragma unroll
-					for (int m = 0; m < M; ++m) w[d][m] = D::phi64(__dadd_rn(dl64[d], (double) (m - sh)));
+				for (int d = 0; d < DIMS; ++d) weights64<D>(dl64[d], w[d]);
 				v = 0.0;
 #pragma unroll
 				for (int e = 0; e < P::V; ++e) {
