@@ -108,20 +108,11 @@ __device__ __forceinline__ void copy_to_shared(T* dst, const T* src)
 // counts) and each block iteration bins one chunk, so the instance is found
 // by one search per chunk and its geometry read from a shared-memory copy.
 // spread: bin by the spread tiles (else the interpolation tiles); moved:
-// positions xn (else x); forces: 1 = fl, 2 = fs (the bins' force
-// statistics for the FP32C scale, see BinStats), 0 = none.
-template <int DIMS>
-__device__ __forceinline__ void instance_forces(const BatchInst& si, const BatchIO& so, int forces, int p, float* a)
-{
-	const double* f = forces == 1 ? so.fl : so.fs;
-#pragma unroll
-	for (int c = 0; c < DIMS; ++c) a[c] = fabsf((float) (si.g.res * __ldg(f + (size_t) c * so.n + p)));
-}
-
+// positions xn (else x).
 template <int M, int DIMS>
 __global__ void __launch_bounds__(kBinThreads)
-batch_bin_count_kernel(const BatchInst* __restrict__ insts, BatchTable t, int spread, int moved, int forces,
-                       int* __restrict__ counts, int2* __restrict__ key_rank, unsigned* __restrict__ binmax)
+batch_bin_count_kernel(const BatchInst* __restrict__ insts, BatchTable t, int spread, int moved,
+                       int* __restrict__ counts, int* __restrict__ rank)
 {
 	__shared__ int cur_inst, cur_chunk;
 	__shared__ BatchInst si;
@@ -141,28 +132,27 @@ batch_bin_count_kernel(const BatchInst* __restrict__ insts, BatchTable t, int sp
 		const int p = cur_chunk * kBinThreads + threadIdx.x;
 		const bool active = p < n;
 		int key = 0;
-		float a[kMaxDims] = {0.0f, 0.0f, 0.0f};
 		if (active) {
-			// forces is uniform, and a bound instance with points has its force array
-			if (forces) instance_forces<DIMS>(si, so, forces, p, a);
 			const double* x = moved ? so.xn : so.x;
 			key = spread ? si.bin_s + point_bin<M, DIMS>(si.g, si.ts, x, n, p, nullptr)
 			             : si.bin_i + point_bin<M, DIMS>(si.g, si.ti, x, n, p, nullptr);
 		}
 		const unsigned mask = __ballot_sync(0xffffffffu, active);
-		if (active) bin_rank<DIMS>(mask, key, counts, key_rank + so.pbase + p, forces ? a : nullptr, binmax);
+		if (active) rank[so.pbase + p] = bin_rank(mask, key, counts);
 		__syncthreads();            // the next chunk overwrites the shared copies
 	}
 }
 
 // Records of every bound point at their sorted positions, by the same
-// chunks as the count kernel.
+// chunks as the count kernel; forces: 1 = fl, 2 = fs (in record order, for an
+// FP32C spread, see BinForces), 0 = none.  clear: a word to zero, or null.
 template <int M, int DIMS>
 __global__ void __launch_bounds__(kBinThreads)
-batch_bin_scatter_kernel(const BatchInst* __restrict__ insts, BatchTable t, int spread, int moved,
-                         const int2* __restrict__ key_rank, const int* __restrict__ offset,
-                         PointRec* __restrict__ recs)
+batch_bin_scatter_kernel(const BatchInst* __restrict__ insts, BatchTable t, int spread, int moved, int forces,
+                         const int* __restrict__ rank, const int* __restrict__ offset,
+                         PointRec* __restrict__ recs, float4* __restrict__ fout, int* __restrict__ clear)
 {
+	if (clear != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
 	__shared__ int cur_inst, cur_chunk;
 	__shared__ BatchInst si;
 	__shared__ BatchIO so;
@@ -180,11 +170,16 @@ batch_bin_scatter_kernel(const BatchInst* __restrict__ insts, BatchTable t, int 
 		const int p = cur_chunk * kBinThreads + threadIdx.x;
 		if (p < so.n) {
 			const int gp = so.pbase + p;
-			const int2 kr = __ldg(key_rank + gp);
+			const int at = __ldg(rank + gp);
+			float4 f;
+			// forces is uniform, and a bound instance with points has its force array
+			if (forces) f = point_force<DIMS>(forces == 1 ? so.fl : so.fs, si.g.res, so.n, p);
 			PointRec r;
-			point_bin<M, DIMS>(si.g, spread ? si.ts : si.ti, moved ? so.xn : so.x, so.n, p, &r);
+			const int bin = point_bin<M, DIMS>(si.g, spread ? si.ts : si.ti, moved ? so.xn : so.x, so.n, p, &r);
+			const int slot = __ldg(offset + (spread ? si.bin_s : si.bin_i) + bin) + at;
 			r.p = gp;
-			store_rec(recs + __ldg(offset + kr.x) + kr.y, r);
+			store_rec(recs + slot, r);
+			if (forces) fout[slot] = f;
 		}
 		__syncthreads();            // the next chunk overwrites the shared copies
 	}
@@ -207,8 +202,8 @@ __device__ __forceinline__ void next_item(int* next, int nitems, int nact, const
 template <typename D, int DIMS, int NT = kTileThreads>
 __global__ void __launch_bounds__(NT, 1024 / NT)
 batch_spread_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __restrict__ next,
-                    const PointRec* __restrict__ recs, const int* __restrict__ off, const unsigned* __restrict__ binmax,
-                    int step, Deferral defer)
+                    const PointRec* __restrict__ recs, const float4* __restrict__ forces, const int* __restrict__ off,
+                    Deferral defer)
 {
 	__shared__ int cur_inst, cur_local, cur_item;
 	__shared__ BatchInst si;
@@ -223,10 +218,8 @@ batch_spread_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __re
 		copy_to_shared(&so, t.io + inst);
 		__syncthreads();
 		const CompPtrs& fe = so.fe;
-		const BinStatsView bs{binmax + (size_t) si.bin_s * kMaxDims};
 		// a dense tile is deferred by its work-item index
-		spread_tile<D, DIMS, false, NT>(si.g, si.ts, so.n, step ? so.fs : so.fl, recs, so.pbase, off + si.bin_s, bs, fe,
-		                                local, -1, defer, item);
+		spread_tile<D, DIMS, false, NT>(si.g, si.ts, recs, forces, off + si.bin_s, fe, local, -1, defer, item);
 		__syncthreads();
 	}
 }
@@ -261,7 +254,7 @@ batch_spread64_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __
 template <typename D, int DIMS>
 __global__ void __launch_bounds__(kTileThreads, 4)
 batch_spread_dense_kernel(const BatchInst* __restrict__ insts, BatchTable t, const PointRec* __restrict__ recs,
-                          const int* __restrict__ off, const unsigned* __restrict__ binmax, int step,
+                          const float4* __restrict__ forces, const int* __restrict__ off,
                           const int* __restrict__ list, const int* __restrict__ count)
 {
 	__shared__ BatchInst si;
@@ -283,9 +276,7 @@ batch_spread_dense_kernel(const BatchInst* __restrict__ insts, BatchTable t, con
 		copy_to_shared(&so, t.io + cur_inst);
 		__syncthreads();
 		const CompPtrs& fe = so.fe;
-		const BinStatsView bs{binmax + (size_t) si.bin_s * kMaxDims};
-		spread_tile<D, DIMS, true>(si.g, si.ts, so.n, step ? so.fs : so.fl, recs, so.pbase, off + si.bin_s, bs, fe,
-		                           cur_local, cur_comp);
+		spread_tile<D, DIMS, true>(si.g, si.ts, recs, forces, off + si.bin_s, fe, cur_local, cur_comp);
 		__syncthreads();
 	}
 }
@@ -371,9 +362,9 @@ struct Batch {
 	// scratch
 	int *d_counts = nullptr, *d_off = nullptr, *d_chunk = nullptr, *d_next = nullptr;
 	int* d_status = nullptr;
-	int2* d_kr = nullptr;
+	int* d_rank = nullptr;
 	PointRec* d_recs = nullptr;
-	unsigned* d_binmax = nullptr;               // spread bins' force maxima (FP32C)
+	float4* d_forces = nullptr;                 // the records' forces (FP32C)
 	int* d_defer = nullptr;                     // deferred dense spread items: count, then the list
 	size_t defer_cap = 0;
 	// step parameters and graphs
@@ -425,18 +416,13 @@ ibk_status batch_bin(Batch& b, cudaStream_t s, int spread, int moved, int forces
 {
 	const BatchTable t = table_view(b);
 	const int nbins = spread ? b.bins_s : b.bins_i;
-	if (forces) {
-		ibk_status st = cuda_check(cudaMemsetAsync(b.d_binmax, 0, sizeof(unsigned) * kMaxDims * (size_t) nbins, s),
-		                           "cudaMemsetAsync");
-		if (st != IBK_OK) return st;
-	}
-	batch_bin_count_kernel<M, DIMS><<<b.grid_bin, kBinThreads, 0, s>>>(b.d_inst, t, spread, moved, forces,
-	                                                                    b.d_counts, b.d_kr, b.d_binmax);
 	const int nchunks = (nbins + kScanChunk - 1) / kScanChunk;
+	batch_bin_count_kernel<M, DIMS><<<b.grid_bin, kBinThreads, 0, s>>>(b.d_inst, t, spread, moved, b.d_counts, b.d_rank);
 	bin_chunk_sum_kernel<<<nchunks, kScanThreads, 0, s>>>(b.d_counts, b.d_chunk, nbins);
 	bin_scan_kernel<<<nchunks, kScanThreads, 0, s>>>(b.d_counts, b.d_chunk, b.d_off, nbins, nchunks);
-	batch_bin_scatter_kernel<M, DIMS><<<b.grid_bin, kBinThreads, 0, s>>>(b.d_inst, t, spread, moved, b.d_kr,
-	                                                                      b.d_off, b.d_recs);
+	batch_bin_scatter_kernel<M, DIMS><<<b.grid_bin, kBinThreads, 0, s>>>(b.d_inst, t, spread, moved, forces, b.d_rank,
+	                                                                      b.d_off, b.d_recs, b.d_forces,
+	                                                                      forces ? b.d_defer : nullptr);
 	b.launches += 4;
 	return check_launch("batch binning");
 }
@@ -469,21 +455,19 @@ ibk_status batch_run_impl(Batch& b, int op, cudaStream_t s)
 				b.d_inst, t, b.d_next, b.d_recs, b.d_off, step ? 1 : 0);
 		} else {
 			Deferral defer{b.d_defer + 4, b.d_defer};
-			ibk_status ds = cuda_check(cudaMemsetAsync(b.d_defer, 0, sizeof(int), s), "cudaMemsetAsync");
-			if (ds != IBK_OK) return ds;
 			if (b.config.spread_threads == 512)
 				batch_spread_kernel<D, DIMS, 512><<<b.grid_s, 512, b.smem_s, s>>>(
-					b.d_inst, t, b.d_next, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer);
+					b.d_inst, t, b.d_next, b.d_recs, b.d_forces, b.d_off, defer);
 			else
 				batch_spread_kernel<D, DIMS><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
-					b.d_inst, t, b.d_next, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer);
+					b.d_inst, t, b.d_next, b.d_recs, b.d_forces, b.d_off, defer);
 			batch_spread_dense_kernel<D, DIMS><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
-				b.d_inst, t, b.d_recs, b.d_off, b.d_binmax, step ? 1 : 0, defer.list, defer.count);
+				b.d_inst, t, b.d_recs, b.d_forces, b.d_off, defer.list, defer.count);
 			b.launches += 1;
 		}
 		return check_launch("batch_spread_kernel");
 	};
-	// FP32C spreads take the bins' force statistics from the binning
+	// FP32C spreads take the forces from the binning
 	const int forces = PREC == IBK_PRECISION_FP32C ? (step ? 2 : 1) : 0;
 	if (op == IBK_OP_INTERPOLATE || step) {
 		if ((st = batch_bin<D::M, DIMS>(b, s, 0, 0, 0)) != IBK_OK) return st;
@@ -689,15 +673,14 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 		// bin arrays sized for the larger bin space (counts start zeroed and
 		// every scan leaves them zeroed)
 		void** bufs[] = {reinterpret_cast<void**>(&b.d_counts), reinterpret_cast<void**>(&b.d_off),
-		                 reinterpret_cast<void**>(&b.d_chunk), reinterpret_cast<void**>(&b.d_binmax)};
-		const size_t bytes[] = {sizeof(int) * nb, sizeof(int) * (nb + 1), sizeof(int) * (nb / kScanChunk + 2),
-		                        sizeof(unsigned) * kMaxDims * nb};
+		                 reinterpret_cast<void**>(&b.d_chunk)};
+		const size_t bytes[] = {sizeof(int) * nb, sizeof(int) * (nb + 1), sizeof(int) * (nb / kScanChunk + 2)};
 		b.bins_cap = 0;
-		for (int j = 0; j < 4; ++j) {
+		for (int j = 0; j < 3; ++j) {
 			if (*bufs[j]) cudaFree(*bufs[j]);
 			*bufs[j] = nullptr;
 		}
-		for (int j = 0; j < 4; ++j)
+		for (int j = 0; j < 3; ++j)
 			if ((st = cuda_check(cudaMalloc(bufs[j], bytes[j]), "cudaMalloc")) != IBK_OK) return st;
 		if ((st = cuda_check(cudaMemset(b.d_counts, 0, bytes[0]), "cudaMemset")) != IBK_OK) return st;
 		b.bins_cap = nb;
@@ -751,7 +734,7 @@ void destroy(Batch* b)
 		if (b->h_ring[r]) cudaFreeHost(b->h_ring[r]);
 	}
 	void* bufs[] = {b->d_inst, b->d_table, b->d_counts, b->d_off, b->d_chunk, b->d_recs,
-	                b->d_next, b->d_status, b->d_kr, b->d_binmax, b->d_defer};
+	                b->d_next, b->d_status, b->d_rank, b->d_forces, b->d_defer};
 	for (void* p : bufs)
 		if (p) cudaFree(p);
 	if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
@@ -852,7 +835,9 @@ ibk_status ibk_batch_create(int count, const ibk_instance_desc* instances, ibk_d
 	}
 	const size_t pts = (size_t) std::max(max_points, 1);
 	cap = 0;
-	if (st == IBK_OK) st = grow(&b->d_kr, cap, pts, "cudaMalloc");
+	if (st == IBK_OK) st = grow(&b->d_rank, cap, pts, "cudaMalloc");
+	cap = 0;
+	if (st == IBK_OK && precision == IBK_PRECISION_FP32C) st = grow(&b->d_forces, cap, pts, "cudaMalloc");
 	cap = 0;
 	if (st == IBK_OK) st = grow(&b->d_recs, cap, pts, "cudaMalloc");
 	cap = 0;

@@ -17,9 +17,11 @@
 // read records contiguously, bin after bin, and never redo the FP64 step in
 // the FP32C form (the FP64 form redoes it for its exact weights only).
 //
-//   bin_count_kernel    key = tile * 3^dims + class; warp-aggregated rank
+//   bin_count_kernel    key = tile * 3^dims + class; warp-aggregated rank; its
+//                       last block scans the counts where they are few
 //   bin_scan_kernel     exclusive scan of the bin counts (resets the counts)
-//   bin_scatter_kernel  records[offset[key] + rank] = record of the point
+//   bin_scatter_kernel  records[offset[key] + rank] = record of the point, and
+//                       for an FP32C spread its forces in the same order
 // The non-template kernels are static: each translation unit that launches
 // them carries its own copy.
 #pragma once
@@ -137,30 +139,9 @@ __device__ __forceinline__ int point_bin(const GridGeom& g, const TileGeom& tg, 
 	return tile * tg.nclass + cls;
 }
 
-// Force statistics of the bins (spread only): binmax[bin * 3 + c] = the
-// largest |f| of the bin's points as FP32 bits (f = FP32 res * F_c, the value
-// the FP32C spread multiplies), from which a tile takes the largest term its
-// fixed point must hold.  An integer maximum: independent of the order of
-// the atomics (the binning order is not deterministic; this is).
-struct BinStats {
-	const double* f;        // forces (dims * n), nullptr: no statistics
-	double res;             // product of the resolutions (1 / h^dims)
-	unsigned* binmax;
-};
-
-template <int DIMS>
-__device__ __forceinline__ void force_abs(const BinStats& st, int n, int p, float* a)
-{
-#pragma unroll
-	for (int c = 0; c < DIMS; ++c) a[c] = fabsf((float) (st.res * __ldg(st.f + (size_t) c * n + p)));
-}
-
 // Warp-aggregated rank of a point in its bin: one atomic per group of lanes
-// sharing a key; with statistics (a != nullptr) also the group's largest
-// |f| per component.  Every lane of `mask` must call it.
-template <int DIMS>
-__device__ __forceinline__ void bin_rank(unsigned mask, int key, int* __restrict__ count, int2* __restrict__ kr_out,
-                                         const float* a, unsigned* __restrict__ binmax)
+// sharing a key.  Every lane of `mask` must call it.
+__device__ __forceinline__ int bin_rank(unsigned mask, int key, int* __restrict__ count)
 {
 	const int lane = threadIdx.x & 31;
 	const unsigned peers = __match_any_sync(mask, key);
@@ -168,29 +149,7 @@ __device__ __forceinline__ void bin_rank(unsigned mask, int key, int* __restrict
 	int base = 0;
 	if (lane == leader) base = atomicAdd(count + key, __popc(peers));
 	base = __shfl_sync(peers, base, leader);
-	*kr_out = make_int2(key, base + __popc(peers & ((1u << lane) - 1u)));
-	if (a != nullptr) {
-#pragma unroll
-		for (int c = 0; c < DIMS; ++c) {
-			const unsigned m = __reduce_max_sync(peers, __float_as_uint(a[c]));
-			if (lane == leader && m != 0u) atomicMax(binmax + (size_t) key * kMaxDims + c, m);
-		}
-	}
-}
-
-template <int M, int DIMS>
-__global__ void __launch_bounds__(256)
-bin_count_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
-                 int* __restrict__ count, int2* __restrict__ key_rank, BinStats st)
-{
-	const int p = blockIdx.x * blockDim.x + threadIdx.x;
-	const bool active = p < n;
-	float a[kMaxDims] = {0.0f, 0.0f, 0.0f};
-	if (st.f != nullptr && active) force_abs<DIMS>(st, n, p, a);   // loads in flight with x's
-	const int key = active ? point_bin<M, DIMS>(g, tg, x, n, p, nullptr) : 0;
-	const unsigned mask = __ballot_sync(0xffffffffu, active);
-	if (!active) return;
-	bin_rank<DIMS>(mask, key, count, key_rank + p, st.f != nullptr ? a : nullptr, st.binmax);
+	return base + __popc(peers & ((1u << lane) - 1u));
 }
 
 // Exclusive scan of the bin counts in two launches.  Each CTA owns a chunk
@@ -226,6 +185,68 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int& total)
 	const int r = (warp ? warp_sums[warp - 1] : 0) + incl - v;
 	__syncthreads();
 	return r;
+}
+
+// The scan by the last block of a count kernel (with TAIL) to finish; ticket: 0
+// before the launch and after it.  Up to kTailBins bins it is one step of the
+// block and saves the two launches of the scan, about 5 us; with 13,824 bins
+// (four steps) it cost 13 us more than they do.
+constexpr int kTailBins = 4096;
+
+struct ScanTail {
+	int* offset;
+	unsigned* ticket;
+	int num_bins;
+};
+
+// Every thread of a 256-thread block calls it, done with its atomics on count.
+__device__ __forceinline__ void scan_tail(const ScanTail& t, int* __restrict__ count)
+{
+	constexpr int kPer = 16;
+	__shared__ bool last;
+	__threadfence();
+	__syncthreads();
+	if (threadIdx.x == 0) last = atomicAdd(t.ticket, 1u) == gridDim.x - 1u;
+	__syncthreads();
+	if (!last) return;
+	__threadfence();
+	int carry = 0;
+	for (int b0 = 0; b0 < t.num_bins; b0 += 256 * kPer) {
+		const int i0 = b0 + threadIdx.x * kPer;
+		int v[kPer], sum = 0, total;
+#pragma unroll
+		for (int q = 0; q < kPer; ++q) {
+			v[q] = i0 + q < t.num_bins ? __ldcg(count + i0 + q) : 0;
+			sum += v[q];
+		}
+		int run = carry + block_exclusive_scan(sum, total);
+#pragma unroll
+		for (int q = 0; q < kPer; ++q) {
+			if (i0 + q < t.num_bins) {
+				t.offset[i0 + q] = run;
+				count[i0 + q] = 0;
+			}
+			run += v[q];
+		}
+		carry += total;
+	}
+	if (threadIdx.x == 0) {
+		t.offset[t.num_bins] = carry;
+		*t.ticket = 0u;
+	}
+}
+
+template <int M, int DIMS, bool TAIL>
+__global__ void __launch_bounds__(256)
+bin_count_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
+                 int* __restrict__ count, int* __restrict__ rank, ScanTail tail)
+{
+	const int p = blockIdx.x * blockDim.x + threadIdx.x;
+	const bool active = p < n;
+	const int key = active ? point_bin<M, DIMS>(g, tg, x, n, p, nullptr) : 0;
+	const unsigned mask = __ballot_sync(0xffffffffu, active);
+	if (active) rank[p] = bin_rank(mask, key, count);
+	if constexpr (TAIL) scan_tail(tail, count);
 }
 
 static __global__ void __launch_bounds__(kScanThreads)
@@ -279,22 +300,45 @@ bin_scan_kernel(int* __restrict__ count, const int* __restrict__ chunk, int* __r
 	if (blockIdx.x == nchunks - 1 && threadIdx.x == kScanThreads - 1) offset[num_bins] = run;
 }
 
+// Forces of the binned points for an FP32C spread: (float) (res * F) per
+// component, in record order: the spread reads them beside the records and
+// takes each tile's largest force from them.  (Gathered from the input order,
+// with the bins' maxima from atomics of the count kernel, the count took 344
+// and the scatter 220 us for 10.9 M points; now 217 and 296.)
+struct BinForces {
+	const double* f;        // dims * n; null: no forces
+	double res;             // product of the resolutions (1 / h^dims)
+	float4* out;
+};
+
+template <int DIMS>
+__device__ __forceinline__ float4 point_force(const double* __restrict__ f, double res, int n, int p)
+{
+	return make_float4((float) (res * __ldg(f + p)), (float) (res * __ldg(f + (size_t) n + p)),
+	                   DIMS == 3 ? (float) (res * __ldg(f + 2 * (size_t) n + p)) : 0.0f, 0.0f);
+}
+
 // The record of every point at its sorted position (the FP64 index step is
 // recomputed here rather than stored by the count kernel: it costs less
-// than writing and re-reading the records in input order).
+// than writing and re-reading the records in input order).  clear: a word to
+// zero for a later kernel, or null.
 template <int M, int DIMS>
 __global__ void __launch_bounds__(256)
 bin_scatter_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
-                   const int2* __restrict__ key_rank, const int* __restrict__ offset,
-                   PointRec* __restrict__ recs)
+                   const int* __restrict__ rank, const int* __restrict__ offset,
+                   PointRec* __restrict__ recs, BinForces bf, int* __restrict__ clear)
 {
 	const int p = blockIdx.x * blockDim.x + threadIdx.x;
+	if (clear != nullptr && p == 0) *clear = 0;
 	if (p >= n) return;
-	const int2 kr = __ldg(key_rank + p);
+	float4 f;
+	if (bf.f != nullptr) f = point_force<DIMS>(bf.f, bf.res, n, p);     // loads in flight with x's
+	const int at = __ldg(rank + p);
 	PointRec r;
-	point_bin<M, DIMS>(g, tg, x, n, p, &r);
+	const int slot = __ldg(offset + point_bin<M, DIMS>(g, tg, x, n, p, &r)) + at;
 	r.p = p;
-	store_rec(recs + __ldg(offset + kr.x) + kr.y, r);
+	store_rec(recs + slot, r);
+	if (bf.f != nullptr) bf.out[slot] = f;
 }
 
 } // namespace ibk

@@ -81,7 +81,7 @@ ibk_status launch(Plan& plan, const char* name, cudaStream_t stream, F&& body)
 }
 
 // Scratch slots of a plan.
-enum { kSlotCount = 0, kSlotOffset = 1, kSlotKeyRank = 2, kSlotRecs = 3, kSlotChunk = 4, kSlotBinMax = 5,
+enum { kSlotCount = 0, kSlotOffset = 1, kSlotRank = 2, kSlotRecs = 3, kSlotChunk = 4, kSlotForces = 5,
        kSlotSums = 6, kSlotDefer = 7 };
 
 // Largest tile extent in cells per axis (point records keep tile-relative

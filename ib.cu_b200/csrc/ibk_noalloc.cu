@@ -8,7 +8,7 @@
 // where a cudaMalloc (which synchronises the device) would stall the step,
 // or hosts that never hold a plan at all.  This entry point takes the grid
 // description directly, allocates nothing, and keeps its scratch in one
-// file-scope __device__ array of fixed size (kNoallocBytes, about 22 MB),
+// file-scope __device__ array of fixed size (kNoallocBytes, about 20 MB),
 // which every GPU that loads this library holds until the process exits.
 //
 // Limits: at most kNoallocMaxPoints points and kNoallocMaxBins bins
@@ -37,8 +37,8 @@ constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kOffCount = 0;
 constexpr size_t kOffOffset = kOffCount + align256(sizeof(int) * kNoallocMaxBins);
 constexpr size_t kOffChunk = kOffOffset + align256(sizeof(int) * (kNoallocMaxBins + 1));
-constexpr size_t kOffKeyRank = kOffChunk + align256(sizeof(int) * kNoallocMaxChunks);
-constexpr size_t kOffRecs = kOffKeyRank + align256(sizeof(int2) * kNoallocMaxPoints);
+constexpr size_t kOffRank = kOffChunk + align256(sizeof(int) * kNoallocMaxChunks);
+constexpr size_t kOffRecs = kOffRank + align256(sizeof(int) * kNoallocMaxPoints);
 constexpr size_t kNoallocBytes = kOffRecs + align256(sizeof(PointRec) * kNoallocMaxPoints);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
@@ -123,7 +123,7 @@ ibk_status run(const GridGeom& g, int tag, int n, const double* x, ConstCompPtrs
 	int* count = reinterpret_cast<int*>(base + kOffCount);
 	int* off = reinterpret_cast<int*>(base + kOffOffset);
 	int* chunk = reinterpret_cast<int*>(base + kOffChunk);
-	int2* kr = reinterpret_cast<int2*>(base + kOffKeyRank);
+	int* rank = reinterpret_cast<int*>(base + kOffRank);
 	PointRec* recs = reinterpret_cast<PointRec*>(base + kOffRecs);
 	// the array keeps the previous call's contents: clear what must start at 0
 	// (the bin counts; everything else is written before it is read)
@@ -131,14 +131,14 @@ ibk_status run(const GridGeom& g, int tag, int n, const double* x, ConstCompPtrs
 	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
 	const int nb = (n + 255) / 256;
 	const int nchunks = (tg.num_bins + kScanChunk - 1) / kScanChunk;
-	const BinStats no_stats{nullptr, g.res, nullptr};   // interpolation: no force statistics
-	bin_count_kernel<M, DIMS><<<nb, 256, 0, stream>>>(g, tg, n, x, count, kr, no_stats);
+	bin_count_kernel<M, DIMS, false><<<nb, 256, 0, stream>>>(g, tg, n, x, count, rank, ScanTail{off, nullptr, tg.num_bins});
 	if ((s = check_launch("bin_count_kernel")) != IBK_OK) return s;
 	bin_chunk_sum_kernel<<<nchunks, kScanThreads, 0, stream>>>(count, chunk, tg.num_bins);
 	if ((s = check_launch("bin_chunk_sum_kernel")) != IBK_OK) return s;
 	bin_scan_kernel<<<nchunks, kScanThreads, 0, stream>>>(count, chunk, off, tg.num_bins, nchunks);
 	if ((s = check_launch("bin_scan_kernel")) != IBK_OK) return s;
-	bin_scatter_kernel<M, DIMS><<<nb, 256, 0, stream>>>(g, tg, n, x, kr, off, recs);
+	bin_scatter_kernel<M, DIMS><<<nb, 256, 0, stream>>>(g, tg, n, x, rank, off, recs, BinForces{nullptr, g.res, nullptr},
+	                                                       nullptr);
 	if ((s = check_launch("bin_scatter_kernel")) != IBK_OK) return s;
 	const size_t smem = interp_smem_bytes<M>(g, tg);
 	auto kern = interp_tile_kernel<D, DIMS, PREC>;

@@ -42,52 +42,68 @@ ibk_status interp_direct(Plan& plan, const OpArgs& a, ConstCompPtrs ue, double* 
 	});
 }
 
-// Counting sort of the points by (tile, reach class): records in bin order
-// and the bin offsets; with forces f (a spread follows) also the bins' force
-// statistics for the FP32C scale.
+// What the binning leaves: records in bin order, the bin offsets and, for an
+// FP32C spread, the points' forces beside the records and the deferral list
+// with its count zeroed.
+struct Binned {
+	const PointRec* recs = nullptr;
+	const int* off = nullptr;
+	const float4* forces = nullptr;
+	Deferral defer{nullptr, nullptr};
+};
+
+// Counting sort of the points by (tile, reach class); f: the forces an FP32C
+// spread of these points takes, or null.
 template <int M, int DIMS>
-ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, const PointRec** recs_out,
-                      const int** off_out, const double* f = nullptr, BinStatsView* stats_out = nullptr)
+ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, Binned& out, const double* f = nullptr)
 {
 	ibk_status s;
 	const int need = a.n > plan.reserved_points ? a.n : plan.reserved_points;
 	if ((s = ensure_scratch(plan, kSlotCount, sizeof(int) * (size_t) tg.num_bins, a.stream, true)) != IBK_OK) return s;
 	if ((s = ensure_scratch(plan, kSlotOffset, sizeof(int) * ((size_t) tg.num_bins + 1), a.stream)) != IBK_OK) return s;
-	if ((s = ensure_scratch(plan, kSlotKeyRank, sizeof(int2) * (size_t) need, a.stream)) != IBK_OK) return s;
+	if ((s = ensure_scratch(plan, kSlotRank, sizeof(int) * (size_t) need, a.stream)) != IBK_OK) return s;
 	if ((s = ensure_scratch(plan, kSlotRecs, sizeof(PointRec) * (size_t) need, a.stream)) != IBK_OK) return s;
 	const int nchunks = (tg.num_bins + kScanChunk - 1) / kScanChunk;
-	if ((s = ensure_scratch(plan, kSlotChunk, sizeof(int) * ((size_t) nchunks + 1), a.stream)) != IBK_OK) return s;
+	// the count kernel's ticket, then the chunk sums
+	if ((s = ensure_scratch(plan, kSlotChunk, sizeof(int) * ((size_t) nchunks + 2), a.stream, true)) != IBK_OK) return s;
 	int* count = static_cast<int*>(plan.scratch[kSlotCount].ptr);
 	int* off = static_cast<int*>(plan.scratch[kSlotOffset].ptr);
-	int2* kr = static_cast<int2*>(plan.scratch[kSlotKeyRank].ptr);
+	int* rank = static_cast<int*>(plan.scratch[kSlotRank].ptr);
 	PointRec* recs = static_cast<PointRec*>(plan.scratch[kSlotRecs].ptr);
-	int* chunk = static_cast<int*>(plan.scratch[kSlotChunk].ptr);
+	unsigned* ticket = static_cast<unsigned*>(plan.scratch[kSlotChunk].ptr);
+	int* chunk = static_cast<int*>(plan.scratch[kSlotChunk].ptr) + 1;
 	const GridGeom& g = *a.g;
 	const int nb = blocks_for(a.n, 256);
-	BinStats st{nullptr, g.res, nullptr};
+	BinForces bf{f, g.res, nullptr};
+	int* clear = nullptr;
 	if (f) {
-		const size_t nm = sizeof(unsigned) * kMaxDims * (size_t) tg.num_bins;
-		if ((s = ensure_scratch(plan, kSlotBinMax, nm, a.stream)) != IBK_OK) return s;
-		st.f = f;
-		st.binmax = static_cast<unsigned*>(plan.scratch[kSlotBinMax].ptr);
-		cudaError_t e = cudaMemsetAsync(st.binmax, 0, nm, a.stream);
-		if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-		*stats_out = BinStatsView{st.binmax};
+		if ((s = ensure_scratch(plan, kSlotForces, sizeof(float4) * (size_t) need, a.stream)) != IBK_OK) return s;
+		if ((s = ensure_scratch(plan, kSlotDefer, sizeof(int) * ((size_t) tg.num_tiles * DIMS + 4), a.stream)) != IBK_OK)
+			return s;
+		bf.out = static_cast<float4*>(plan.scratch[kSlotForces].ptr);
+		clear = static_cast<int*>(plan.scratch[kSlotDefer].ptr);
+		out.forces = bf.out;
+		out.defer = Deferral{clear + 4, clear};
 	}
+	const bool tail = tg.num_bins <= kTailBins;
+	const ScanTail scan{off, ticket, tg.num_bins};
 	if ((s = launch(plan, "bin_count_kernel", a.stream, [&] {
-		bin_count_kernel<M, DIMS><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, count, kr, st);
+		if (tail) bin_count_kernel<M, DIMS, true><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, count, rank, scan);
+		else bin_count_kernel<M, DIMS, false><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, count, rank, scan);
 	})) != IBK_OK) return s;
-	if ((s = launch(plan, "bin_chunk_sum_kernel", a.stream, [&] {
-		bin_chunk_sum_kernel<<<nchunks, kScanThreads, 0, a.stream>>>(count, chunk, tg.num_bins);
-	})) != IBK_OK) return s;
-	if ((s = launch(plan, "bin_scan_kernel", a.stream, [&] {
-		bin_scan_kernel<<<nchunks, kScanThreads, 0, a.stream>>>(count, chunk, off, tg.num_bins, nchunks);
-	})) != IBK_OK) return s;
+	if (!tail) {
+		if ((s = launch(plan, "bin_chunk_sum_kernel", a.stream, [&] {
+			bin_chunk_sum_kernel<<<nchunks, kScanThreads, 0, a.stream>>>(count, chunk, tg.num_bins);
+		})) != IBK_OK) return s;
+		if ((s = launch(plan, "bin_scan_kernel", a.stream, [&] {
+			bin_scan_kernel<<<nchunks, kScanThreads, 0, a.stream>>>(count, chunk, off, tg.num_bins, nchunks);
+		})) != IBK_OK) return s;
+	}
 	if ((s = launch(plan, "bin_scatter_kernel", a.stream, [&] {
-		bin_scatter_kernel<M, DIMS><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, kr, off, recs);
+		bin_scatter_kernel<M, DIMS><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, rank, off, recs, bf, clear);
 	})) != IBK_OK) return s;
-	*recs_out = recs;
-	*off_out = off;
+	out.recs = recs;
+	out.off = off;
 	return IBK_OK;
 }
 
@@ -102,8 +118,7 @@ ibk_status set_smem(K kernel, size_t bytes)
 }
 
 template <typename D, int DIMS, int PREC>
-ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const PointRec* recs, const int* off,
-                         BinStatsView bs, const double* fl, CompPtrs fe)
+ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const Binned& b, const double* fl, CompPtrs fe)
 {
 	const size_t smem = spread_smem_bytes(*a.g, tg, D::M, PREC);
 	ibk_status s;
@@ -121,7 +136,8 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 			if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
 		}
 		return launch(plan, "spread_tile_kernel", a.stream, [&] {
-			kern<<<dim3(tg.num_tiles, DIMS, parts), s64_threads<DIMS>(), smem, a.stream>>>(*a.g, tg, a.n, a.x, fl, recs, off, fe);
+			kern<<<dim3(tg.num_tiles, DIMS, parts), s64_threads<DIMS>(), smem, a.stream>>>(*a.g, tg, a.n, a.x, fl, b.recs,
+			                                                                              b.off, fe);
 		});
 	} else {
 		// one CTA per tile for every component, dense tiles deferred to the
@@ -129,18 +145,14 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 		auto kern = spread_tile_kernel<D, DIMS>;
 		auto dense = spread_dense_kernel<D, DIMS>;
 		if ((s = set_smem(kern, smem)) != IBK_OK || (s = set_smem(dense, smem)) != IBK_OK) return s;
-		if ((s = ensure_scratch(plan, kSlotDefer, sizeof(int) * ((size_t) tg.num_tiles * DIMS + 4), a.stream)) != IBK_OK)
-			return s;
-		int* count = static_cast<int*>(plan.scratch[kSlotDefer].ptr);
-		const Deferral defer{count + 4, count};
-		cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), a.stream);
-		if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
 		if ((s = launch(plan, "spread_tile_kernel", a.stream, [&] {
-			kern<<<tg.num_tiles, kTileThreads, smem, a.stream>>>(*a.g, tg, a.n, fl, recs, off, bs, fe, defer);
+			kern<<<tg.num_tiles, kTileThreads, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer);
 		})) != IBK_OK) return s;
+		// no face can receive more terms than there are points
+		if (a.n <= 2 * kFoldChunk) return IBK_OK;
 		const int gd = std::max(1, std::min(tg.num_tiles * DIMS, 4 * plan.num_sms));
 		return launch(plan, "spread_dense_kernel", a.stream, [&] {
-			dense<<<gd, kTileThreads, smem, a.stream>>>(*a.g, tg, a.n, fl, recs, off, bs, fe, defer.list, defer.count);
+			dense<<<gd, kTileThreads, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer.list, b.defer.count);
 		});
 	}
 }
@@ -150,13 +162,11 @@ ibk_status spread_impl(Plan& plan, const OpArgs& a, const double* fl, CompPtrs f
 {
 	using D = Delta<KIND, ORDER>;
 	if (!plan.tiled) return spread_direct<D, DIMS>(plan, a, fl, fe);
-	const PointRec* recs = nullptr;
-	const int* off = nullptr;
-	BinStatsView bs{nullptr};
+	Binned b;
 	constexpr bool fix = PREC == IBK_PRECISION_FP32C;
-	ibk_status s = bin_points<D::M, DIMS>(plan, a, plan.spread_tiles, &recs, &off, fix ? fl : nullptr, &bs);
+	ibk_status s = bin_points<D::M, DIMS>(plan, a, plan.spread_tiles, b, fix ? fl : nullptr);
 	if (s != IBK_OK) return s;
-	return launch_spread<D, DIMS, PREC>(plan, a, plan.spread_tiles, recs, off, bs, fl, fe);
+	return launch_spread<D, DIMS, PREC>(plan, a, plan.spread_tiles, b, fl, fe);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -211,8 +221,7 @@ bool grid_tensor_map(CUtensorMap* map, const double* base, const CompGeom& cg, i
 namespace {
 
 template <typename D, int DIMS, int PREC>
-ibk_status launch_interp(Plan& plan, const OpArgs& a, const TileGeom& tg, const PointRec* recs, const int* off,
-                         ConstCompPtrs ue, double* ul)
+ibk_status launch_interp(Plan& plan, const OpArgs& a, const TileGeom& tg, const Binned& b, ConstCompPtrs ue, double* ul)
 {
 	const GridGeom& g = *a.g;
 	const size_t smem = interp_smem_bytes<D::M>(g, tg);
@@ -229,7 +238,7 @@ ibk_status launch_interp(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 	ibk_status s = set_smem(kern, smem);
 	if (s != IBK_OK) return s;
 	return launch(plan, "interp_tile_kernel", a.stream, [&] {
-		kern<<<dim3(tg.num_tiles, DIMS), kTileThreads, smem, a.stream>>>(g, tg, a.n, a.x, recs, off, ue, ul,
+		kern<<<dim3(tg.num_tiles, DIMS), kTileThreads, smem, a.stream>>>(g, tg, a.n, a.x, b.recs, b.off, ue, ul,
 		                                                                   maps, use_tma, plan.d_status);
 	});
 }
@@ -239,11 +248,10 @@ ibk_status interp_impl(Plan& plan, const OpArgs& a, ConstCompPtrs ue, double* ul
 {
 	using D = Delta<KIND, ORDER>;
 	if (!plan.tiled) return interp_direct<D, DIMS>(plan, a, ue, ul);
-	const PointRec* recs = nullptr;
-	const int* off = nullptr;
-	ibk_status s = bin_points<D::M, DIMS>(plan, a, plan.tiles, &recs, &off);
+	Binned b;
+	ibk_status s = bin_points<D::M, DIMS>(plan, a, plan.tiles, b);
 	if (s != IBK_OK) return s;
-	return launch_interp<D, DIMS, PREC>(plan, a, plan.tiles, recs, off, ue, ul);
+	return launch_interp<D, DIMS, PREC>(plan, a, plan.tiles, b, ue, ul);
 }
 
 bool same_tiles(const TileGeom& a, const TileGeom& b)
@@ -261,17 +269,15 @@ ibk_status both_impl(Plan& plan, const OpArgs& a, const double* fl, CompPtrs fe,
 		ibk_status s = spread_direct<D, DIMS>(plan, a, fl, fe);
 		return s != IBK_OK ? s : interp_direct<D, DIMS>(plan, a, ue, ul);
 	}
-	const PointRec* recs = nullptr;
-	const int* off = nullptr;
-	BinStatsView bs{nullptr};
+	Binned b;
 	constexpr bool fix = PREC == IBK_PRECISION_FP32C;
-	ibk_status s = bin_points<D::M, DIMS>(plan, a, plan.spread_tiles, &recs, &off, fix ? fl : nullptr, &bs);
+	ibk_status s = bin_points<D::M, DIMS>(plan, a, plan.spread_tiles, b, fix ? fl : nullptr);
 	if (s != IBK_OK) return s;
-	if ((s = launch_spread<D, DIMS, PREC>(plan, a, plan.spread_tiles, recs, off, bs, fl, fe)) != IBK_OK) return s;
+	if ((s = launch_spread<D, DIMS, PREC>(plan, a, plan.spread_tiles, b, fl, fe)) != IBK_OK) return s;
 	if (!same_tiles(plan.spread_tiles, plan.tiles)) {
-		if ((s = bin_points<D::M, DIMS>(plan, a, plan.tiles, &recs, &off)) != IBK_OK) return s;
+		if ((s = bin_points<D::M, DIMS>(plan, a, plan.tiles, b)) != IBK_OK) return s;
 	}
-	return launch_interp<D, DIMS, PREC>(plan, a, plan.tiles, recs, off, ue, ul);
+	return launch_interp<D, DIMS, PREC>(plan, a, plan.tiles, b, ue, ul);
 }
 
 template <int KIND, int ORDER, int DIMS>

@@ -93,22 +93,14 @@ struct RangeTable {
 	int count;
 };
 
-// The bins' force maxima of a grid for the FP32C scale (see BinStats), or
-// null.
-struct BinStatsView {
-	const unsigned* binmax;
-};
-
 template <int DIMS>
 __device__ __forceinline__ void build_ranges(const GridGeom& g, const TileGeom& tg, const int* tc,
-                                             const int* __restrict__ off, RangeTable& rt,
-                                             BinStatsView bs = BinStatsView{nullptr}, unsigned* fmax = nullptr)
+                                             const int* __restrict__ off, RangeTable& rt)
 {
 	constexpr int nent = DIMS == 3 ? 125 : 25;
 	const int tid = threadIdx.x;
 	int len = 0, st = 0;
 	unsigned sft = 0;
-	int sbin = -1;          // the bin whose statistics this thread contributes
 	if (tid < nent) {
 		int tile = 0, cls = 0, ts = 1, cs = 1;
 		bool ok = true, home = true, first_home = true;
@@ -141,31 +133,11 @@ __device__ __forceinline__ void build_ranges(const GridGeom& g, const TileGeom& 
 				st = __ldg(off + tile * tg.nclass);
 				len = __ldg(off + (tile + 1) * tg.nclass) - st;
 			}
-			sbin = tile * tg.nclass + cls;   // each home class bin once
 		} else if (ok) {
 			const int bin = tile * tg.nclass + cls;
 			st = __ldg(off + bin);
 			len = __ldg(off + bin + 1) - st;
-			sbin = bin;
 		}
-	}
-	if (fmax != nullptr) {
-		// the largest |f| per component over the candidate bins (threads
-		// 0..127 hold one bin each, or none)
-		__shared__ unsigned part_m[4][kMaxDims];
-		unsigned fm[kMaxDims] = {0u, 0u, 0u};
-		if (sbin >= 0)
-#pragma unroll
-			for (int c = 0; c < DIMS; ++c) fm[c] = __ldg(bs.binmax + (size_t) sbin * kMaxDims + c);
-		if (tid < 128)
-#pragma unroll
-			for (int c = 0; c < kMaxDims; ++c) {
-				const unsigned m = __reduce_max_sync(0xffffffffu, fm[c]);
-				if ((tid & 31) == 0) part_m[tid >> 5][c] = m;
-			}
-		__syncthreads();
-		if (tid < kMaxDims)
-			fmax[tid] = max(max(part_m[0][tid], part_m[1][tid]), max(part_m[2][tid], part_m[3][tid]));
 	}
 	// compaction: slot = number of non-empty entries before this one, pref =
 	// exclusive sum of the lengths (the first 128 threads, 4 warps)
@@ -221,8 +193,7 @@ __device__ __forceinline__ int range_walk(const RangeTable& rt, int& r, int item
 
 // Fixed point of the FP32C spread.  Per (tile, component) a power-of-two
 // scale is chosen so that every single |term| stays below 2^22, the largest
-// term being max|w| * max|f| over the candidate bins (the binning's bin
-// maxima, BinStats).  Each FP32 product is scaled, rounded once to an integer
+// term being max|w| * max|f| over the candidates.  Each FP32 product is scaled, rounded once to an integer
 // with the float magic number 1.5 * 2^23 (x + magic carries rint(x) in its
 // low mantissa bits for |x| <= 2^22: an FFMA and an integer subtract, no
 // conversion instruction) and added to the face's 32-bit word with one
@@ -397,6 +368,34 @@ __device__ __forceinline__ float fix_scale(unsigned fmax_bits, float wmax, int n
 	return ldexpf(1.0f, max(-126, min(k, 126)));
 }
 
+// The largest |f| per component over a tile's candidates, as FP32 bits, in
+// fmax (each by the thread of that index).
+template <int NT>
+__device__ __forceinline__ void force_maxima(const RangeTable& rt, int ncand, const float4* __restrict__ forces,
+                                             unsigned* fmax)
+{
+	__shared__ unsigned part[NT / 32][kMaxDims];
+	unsigned m[kMaxDims] = {0u, 0u, 0u};
+	int r = 0;
+	for (int it = threadIdx.x; it < ncand; it += NT) {
+		const float4 f = __ldg(forces + range_walk(rt, r, it));
+		m[0] = max(m[0], __float_as_uint(fabsf(f.x)));
+		m[1] = max(m[1], __float_as_uint(fabsf(f.y)));
+		m[2] = max(m[2], __float_as_uint(fabsf(f.z)));
+	}
+#pragma unroll
+	for (int c = 0; c < kMaxDims; ++c) {
+		m[c] = __reduce_max_sync(0xffffffffu, m[c]);
+		if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][c] = m[c];
+	}
+	__syncthreads();
+	if (threadIdx.x < kMaxDims) {
+		unsigned best = 0u;
+		for (int w = 0; w < NT / 32; ++w) best = max(best, part[w][threadIdx.x]);
+		fmax[threadIdx.x] = best;
+	}
+}
+
 // Shared-memory reduction (no return value) at a 32-bit shared address.
 __device__ __forceinline__ void red_shared(unsigned addr, int v)
 {
@@ -557,9 +556,9 @@ __device__ __forceinline__ void write_tile(double* __restrict__ out, const CompG
 // totals (integers below 2^53) and cleared.  Every thread of the CTA calls
 // it, after s_scale is set.
 template <typename D, int DIMS, int NT>
-__device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const TileGeom& tg, int n,
-                                                const double* __restrict__ fl, const PointRec* __restrict__ recs,
-                                                int pbase, const RangeTable& rt, int ncand, const int* lo,
+__device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const TileGeom& tg,
+                                                const PointRec* __restrict__ recs, const float4* __restrict__ forces,
+                                                const RangeTable& rt, int ncand, const int* lo,
                                                 const int* cells, const bool* wrap, bool wrap_any,
                                                 unsigned acc_addr, const CompPtrs& fe,
                                                 const float* s_scale, int c_lo, int c_hi)
@@ -580,9 +579,9 @@ __device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const Tile
 			int r = 0;
 			for (int chunk = 0; chunk < ncand; chunk += kFoldChunk) {
 				for (int it = chunk + threadIdx.x; it < min(ncand, chunk + kFoldChunk); it += NT) {
-					const PointRec rec = load_rec(recs + range_walk(rt, r, it));
+					const int slot = range_walk(rt, r, it);
+					const PointRec rec = load_rec(recs + slot);
 					const int sft = rt.shift[r];
-					const int p = rec.p - pbase;
 					int l[DIMS];
 					float dl[DIMS];
 #pragma unroll
@@ -591,7 +590,7 @@ __device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const Tile
 						l[d] = rec_origin(rec.org, d) + unpack8(sft, d) + (own ? rec_own_shift(rec.org, d) : 0);
 						dl[d] = own ? rec.dn[d] : rec.dh[d];
 					}
-					const float f = (float) (g.res * __ldg(fl + (size_t) c * n + p)) * sc;
+					const float f = __ldg(reinterpret_cast<const float*>(forces + slot) + c) * sc;
 					if (!wrap_any) {
 						spread_fix<D, DIMS>(acc_addr, l, dl, f, e, ss.S1, ss.S2);
 					} else {
@@ -621,9 +620,8 @@ __device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const Tile
 }
 
 // One FP32C spread tile; every thread of the CTA calls it.  FOLDED takes one
-// component comp of a deferred tile, else every component.  Records carry
-// point indices offset by pbase (a batch numbers the points of all its
-// instances consecutively); off is this grid's bin table.
+// component comp of a deferred tile, else every component.  off is this
+// grid's bin table.
 // Dense tiles (tiles where a face may receive more terms than a 32-bit word
 // holds) are not summed by the one-pass kernel: it appends
 // (defer_id << 2) | c for each component c to the deferral list and leaves
@@ -635,10 +633,9 @@ struct Deferral {
 };
 
 template <typename D, int DIMS, bool FOLDED = false, int NT = kTileThreads>
-__device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& tg, int n,
-                                            const double* __restrict__ fl, const PointRec* __restrict__ recs, int pbase,
-                                            const int* __restrict__ off, BinStatsView bs, const CompPtrs& fe,
-                                            int tile, int comp, Deferral defer = Deferral{nullptr, nullptr},
+__device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& tg, const PointRec* __restrict__ recs,
+                                            const float4* __restrict__ forces, const int* __restrict__ off,
+                                            const CompPtrs& fe, int tile, int comp, Deferral defer = Deferral{nullptr, nullptr},
                                             int defer_id = 0)
 {
 	constexpr int M = D::M;
@@ -664,7 +661,7 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 		wrap_any = wrap_any || wrap[d];
 	}
 	__shared__ unsigned s_fmax[kMaxDims];
-	build_ranges<DIMS>(g, tg, tc, off, rt, bs, s_fmax);
+	build_ranges<DIMS>(g, tg, tc, off, rt);
 	const int ncand = rt.pref[rt.count];
 	if (ncand == 0) {
 		// no point reaches the tile: its faces are zero
@@ -677,9 +674,10 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 		return;
 	}
 	const unsigned acc_addr = smem_addr(acc);
+	force_maxima<NT>(rt, ncand, forces, s_fmax);
 	if constexpr (FOLDED) {
 		if (threadIdx.x < kMaxDims) s_scale[threadIdx.x] = fix_scale(s_fmax[threadIdx.x], max_weight<D, DIMS>(), kFoldChunk);
-		spread_tile_folded<D, DIMS, NT>(g, tg, n, fl, recs, pbase, rt, ncand, lo, cells, wrap, wrap_any, acc_addr,
+		spread_tile_folded<D, DIMS, NT>(g, tg, recs, forces, rt, ncand, lo, cells, wrap, wrap_any, acc_addr,
 		                                fe, s_scale, c_lo, c_hi);
 		return;
 	}
@@ -702,8 +700,8 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 	for (int it = threadIdx.x; it < ncand; it += NT) {
 		const int slot = range_walk(rt, r, it);
 		const PointRec rec = load_rec(recs + slot);
+		const float4 force = __ldg(forces + slot);
 		const int sft = rt.shift[r];
-		const int p = rec.p - pbase;
 		int lh[DIMS];
 #pragma unroll
 		for (int d = 0; d < DIMS; ++d) lh[d] = rec_origin(rec.org, d) + unpack8(sft, d);
@@ -719,7 +717,7 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 			}
 			const float sc = s_scale[c];
 			if (sc == 0.0f) continue;
-			const float f = (float) (g.res * __ldg(fl + (size_t) c * n + p)) * sc;
+			const float f = (c == 0 ? force.x : (c == 1 ? force.y : force.z)) * sc;
 			float dl[DIMS];
 #pragma unroll
 			for (int d = 0; d < DIMS; ++d) dl[d] = (tg.tag_mac && d == c) ? rec.dn[d] : rec.dh[d];
@@ -1081,7 +1079,6 @@ __device__ __forceinline__ void spread_tile64_plane(const GridGeom& g, const Til
 #pragma unroll
 		for (int d = 0; d < 2; ++d) {
 			const int j0 = rec_origin(rec.org, d) + unpack8(sft, d) + (tg.tag_mac && d == c ? rec_own_shift(rec.org, d) : 0) - sh;
-			weights64<D>(axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta, w[d]);
 #pragma unroll
 			for (int m = 0; m < M; ++m) {
 				bool in;
@@ -1089,6 +1086,9 @@ __device__ __forceinline__ void spread_tile64_plane(const GridGeom& g, const Til
 				mk[d] |= (unsigned) in << m;
 			}
 		}
+		if (mk[0] == 0u || mk[1] == 0u) continue;
+#pragma unroll
+		for (int d = 0; d < 2; ++d) weights64<D>(axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta, w[d]);
 		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
 #pragma unroll
 		for (int m1 = 0; m1 < M; ++m1)
@@ -1137,10 +1137,10 @@ __host__ __device__ inline size_t spread_tile_limit_bytes(const GridGeom& g, con
 // accumulators take 54 KB each at 16^3 tiles).
 template <typename D, int DIMS>
 __global__ void __launch_bounds__(kTileThreads, 4)
-spread_tile_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ fl, const PointRec* __restrict__ recs,
-                   const int* __restrict__ off, BinStatsView bs, CompPtrs fe, Deferral defer)
+spread_tile_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, const float4* __restrict__ forces,
+                   const int* __restrict__ off, CompPtrs fe, Deferral defer)
 {
-	spread_tile<D, DIMS>(g, tg, n, fl, recs, 0, off, bs, fe, blockIdx.x, -1, defer, blockIdx.x);
+	spread_tile<D, DIMS>(g, tg, recs, forces, off, fe, blockIdx.x, -1, defer, blockIdx.x);
 }
 
 // grid: (tile, component, part); four CTAs of 52 KB per SM at 16^3 tiles.
@@ -1157,14 +1157,14 @@ spread_tile64_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ 
 // device.
 template <typename D, int DIMS>
 __global__ void __launch_bounds__(kTileThreads, 4)
-spread_dense_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ fl, const PointRec* __restrict__ recs,
-                    const int* __restrict__ off, BinStatsView bs, CompPtrs fe, const int* __restrict__ list,
+spread_dense_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, const float4* __restrict__ forces,
+                    const int* __restrict__ off, CompPtrs fe, const int* __restrict__ list,
                     const int* __restrict__ count)
 {
 	const int m = *count;
 	for (int k = blockIdx.x; k < m; k += gridDim.x) {
 		const int v = __ldg(list + k);
-		spread_tile<D, DIMS, true>(g, tg, n, fl, recs, 0, off, bs, fe, v >> 2, v & 3);
+		spread_tile<D, DIMS, true>(g, tg, recs, forces, off, fe, v >> 2, v & 3);
 		__syncthreads();
 	}
 }
