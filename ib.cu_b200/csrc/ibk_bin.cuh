@@ -341,4 +341,57 @@ bin_scatter_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x,
 	if (bf.f != nullptr) bf.out[slot] = f;
 }
 
+// The whole binning of few points by one block: counts in shared memory, their
+// scan, and each thread's records (at most kSmallPer) kept in registers from
+// the count to the scatter.  Up to kSmallPoints points and kSmallBins bins (one
+// point a thread where the count kernel scans the bins itself): an
+// interpolation of 1,250 points on 64^3 takes 23 instead of 31 us, one red
+// cell's spread and interpolation 73 instead of 80, but 3,500 points 35
+// instead of 33.
+constexpr int kSmallThreads = 1024, kSmallPer = 3;
+constexpr int kSmallPoints = kSmallThreads * kSmallPer, kSmallBins = 24576;
+
+template <int M, int DIMS>
+__global__ void __launch_bounds__(kSmallThreads)
+bin_small_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x, int* __restrict__ offset,
+                 PointRec* __restrict__ recs, BinForces bf, int* __restrict__ clear)
+{
+	extern __shared__ int small_counts[];
+	const int per = (tg.num_bins + kSmallThreads - 1) / kSmallThreads;      // bins a thread scans
+	if (clear != nullptr && threadIdx.x == 0) *clear = 0;
+	for (int i = threadIdx.x; i < tg.num_bins; i += kSmallThreads) small_counts[i] = 0;
+	__syncthreads();
+	PointRec r[kSmallPer];
+	int bin[kSmallPer], rank[kSmallPer];
+#pragma unroll
+	for (int q = 0; q < kSmallPer; ++q) {
+		const int p = q * kSmallThreads + threadIdx.x;
+		bin[q] = -1;
+		if (p >= n) continue;
+		bin[q] = point_bin<M, DIMS>(g, tg, x, n, p, &r[q]);
+		r[q].p = p;
+		rank[q] = atomicAdd(small_counts + bin[q], 1);
+	}
+	__syncthreads();
+	const int b0 = threadIdx.x * per, b1 = min(b0 + per, tg.num_bins);
+	int sum = 0, total;
+	for (int b = b0; b < b1; ++b) sum += small_counts[b];
+	int run = block_exclusive_scan(sum, total);
+	for (int b = b0; b < b1; ++b) {
+		const int c = small_counts[b];
+		small_counts[b] = run;
+		run += c;
+	}
+	__syncthreads();
+	for (int i = threadIdx.x; i < tg.num_bins; i += kSmallThreads) offset[i] = small_counts[i];
+	if (threadIdx.x == 0) offset[tg.num_bins] = total;
+#pragma unroll
+	for (int q = 0; q < kSmallPer; ++q) {
+		if (bin[q] < 0) continue;
+		const int slot = small_counts[bin[q]] + rank[q];
+		store_rec(recs + slot, r[q]);
+		if (bf.f != nullptr) bf.out[slot] = point_force<DIMS>(bf.f, bf.res, n, r[q].p);
+	}
+}
+
 } // namespace ibk

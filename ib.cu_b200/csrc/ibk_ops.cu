@@ -13,6 +13,12 @@ namespace {
 
 constexpr int kThreads = 128;
 
+// Threads of an FP32C spread CTA on grids of at most two tiles per SM, whose
+// time is the candidates per thread (128 x 64 x 128 cells, 124,700 points, 256
+// tiles: 91 -> 82 us; 64^3, 64 tiles: 72 -> 64; at 6 x 12 x 12 tiles and more no
+// difference, and with 1024 threads 94 and 62).
+constexpr int kFewThreads = 512;
+
 // Candidates of an average tile from which the FP64 spread splits them (30^3
 // cells, 416,000 points: 0.71 ms against 1.66 ms with shared atomics).
 constexpr int kS64SplitCandidates = 4096;
@@ -40,6 +46,16 @@ ibk_status interp_direct(Plan& plan, const OpArgs& a, ConstCompPtrs ue, double* 
 	return launch(plan, "interp_direct_kernel", a.stream, [&] {
 		interp_direct_kernel<D, DIMS><<<blocks_for(a.n, kThreads), kThreads, 0, a.stream>>>(*a.g, a.n, a.x, ue, ul);
 	});
+}
+
+// Opt the kernel in to `bytes` of dynamic shared memory (static shared
+// memory counts against the 48 KB default too, so this is always set).
+template <typename K>
+ibk_status set_smem(K kernel, size_t bytes)
+{
+	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
+	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+	return IBK_OK;
 }
 
 // What the binning leaves: records in bin order, the bin offsets and, for an
@@ -85,7 +101,17 @@ ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, Binned& o
 		out.forces = bf.out;
 		out.defer = Deferral{clear + 4, clear};
 	}
+	out.recs = recs;
+	out.off = off;
 	const bool tail = tg.num_bins <= kTailBins;
+	if (a.n <= (tail ? kSmallThreads : kSmallPoints) && tg.num_bins <= kSmallBins) {
+		const size_t smem = sizeof(int) * (size_t) tg.num_bins;
+		auto kern = bin_small_kernel<M, DIMS>;
+		if ((s = set_smem(kern, smem)) != IBK_OK) return s;
+		return launch(plan, "bin_small_kernel", a.stream, [&] {
+			kern<<<1, kSmallThreads, smem, a.stream>>>(g, tg, a.n, a.x, off, recs, bf, clear);
+		});
+	}
 	const ScanTail scan{off, ticket, tg.num_bins};
 	if ((s = launch(plan, "bin_count_kernel", a.stream, [&] {
 		if (tail) bin_count_kernel<M, DIMS, true><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, count, rank, scan);
@@ -102,18 +128,6 @@ ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, Binned& o
 	if ((s = launch(plan, "bin_scatter_kernel", a.stream, [&] {
 		bin_scatter_kernel<M, DIMS><<<nb, 256, 0, a.stream>>>(g, tg, a.n, a.x, rank, off, recs, bf, clear);
 	})) != IBK_OK) return s;
-	out.recs = recs;
-	out.off = off;
-	return IBK_OK;
-}
-
-// Opt the kernel in to `bytes` of dynamic shared memory (static shared
-// memory counts against the 48 KB default too, so this is always set).
-template <typename K>
-ibk_status set_smem(K kernel, size_t bytes)
-{
-	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
-	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
 	return IBK_OK;
 }
 
@@ -142,11 +156,13 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 	} else {
 		// one CTA per tile for every component, dense tiles deferred to the
 		// folded kernel
-		auto kern = spread_tile_kernel<D, DIMS>;
+		const bool few = tg.num_tiles <= 2 * plan.num_sms;
+		auto kern = few ? spread_tile_kernel<D, DIMS, kFewThreads> : spread_tile_kernel<D, DIMS>;
+		const int nt = few ? kFewThreads : kTileThreads;
 		auto dense = spread_dense_kernel<D, DIMS>;
 		if ((s = set_smem(kern, smem)) != IBK_OK || (s = set_smem(dense, smem)) != IBK_OK) return s;
 		if ((s = launch(plan, "spread_tile_kernel", a.stream, [&] {
-			kern<<<tg.num_tiles, kTileThreads, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer);
+			kern<<<tg.num_tiles, nt, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer);
 		})) != IBK_OK) return s;
 		// no face can receive more terms than there are points
 		if (a.n <= 2 * kFoldChunk) return IBK_OK;

@@ -413,9 +413,10 @@ __device__ __forceinline__ void red_row4(unsigned row, int t0, int t1, int t2, i
 	             :: "r"(row), "r"(t0), "r"(t1), "r"(t2), "r"(t3) : "memory");
 }
 
-// The accumulators start kGuardWords after the dynamic shared memory: a
-// row's out-of-tile columns (zero terms) may fall up to M - 1 words before
-// the first row of the first component.
+// The accumulators start kGuardWords after the dynamic shared memory and end
+// as much before its end: a row's out-of-tile columns (zero terms) may fall up
+// to M - 1 words before the first row of the first component or past the last
+// row of the last.
 constexpr int kGuardWords = 8;
 
 // In-tile node mask of one axis: bit m set when node (j0 + m) lies in [0, e).
@@ -705,7 +706,7 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 		int lh[DIMS];
 #pragma unroll
 		for (int d = 0; d < DIMS; ++d) lh[d] = rec_origin(rec.org, d) + unpack8(sft, d);
-#pragma unroll 1
+#pragma unroll
 		for (int c = 0; c < DIMS; ++c) {
 			const CompGeom& cg = g.comp[c];
 			int l[DIMS], e[DIMS];
@@ -1116,31 +1117,32 @@ __device__ __forceinline__ void spread_any64(const GridGeom& g, const TileGeom& 
 
 // Shared memory of a spread CTA.  FP32C: every component's accumulator words
 // (4 bytes per face; the folded form's words and totals of one component, or
-// the occupancy grid, where larger) and the guard words.
+// the occupancy grid, where larger) between guard words.
 __host__ __device__ inline size_t spread_smem_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
 {
 	if (precision != IBK_PRECISION_FP32C) return spread64_smem_bytes(g, tg, M);
 	const size_t words = (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words;
 	const size_t occ = occupancy_words_rt(g, tg, M), acc = words * 3;
-	return ((acc > occ ? acc : occ) + kGuardWords) * 4;
+	return ((acc > occ ? acc : occ) + 2 * kGuardWords) * 4;
 }
 
 // What a tile shape is held to (at most 200 KB; 8 bytes per face of one
 // component in FP64).
 __host__ __device__ inline size_t spread_tile_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
 {
-	if (precision == IBK_PRECISION_FP32C) return spread_smem_bytes(g, tg, M, precision);
+	if (precision == IBK_PRECISION_FP32C) return spread_smem_bytes(g, tg, M, precision) - 4 * kGuardWords;
 	return (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words * 8 + 4 * kGuardWords;
 }
 
 // 256-thread CTAs capped at 64 registers so that four fit on an SM (their
-// accumulators take 54 KB each at 16^3 tiles).
-template <typename D, int DIMS>
-__global__ void __launch_bounds__(kTileThreads, 4)
+// accumulators take 54 KB each at 16^3 tiles), or on grids of few tiles CTAs
+// of NT threads.
+template <typename D, int DIMS, int NT = kTileThreads>
+__global__ void __launch_bounds__(NT, 1024 / NT)
 spread_tile_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, const float4* __restrict__ forces,
                    const int* __restrict__ off, CompPtrs fe, Deferral defer)
 {
-	spread_tile<D, DIMS>(g, tg, recs, forces, off, fe, blockIdx.x, -1, defer, blockIdx.x);
+	spread_tile<D, DIMS, false, NT>(g, tg, recs, forces, off, fe, blockIdx.x, -1, defer, blockIdx.x);
 }
 
 // grid: (tile, component, part); four CTAs of 52 KB per SM at 16^3 tiles.
