@@ -252,7 +252,7 @@ batch_spread64_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __
 // The deferred dense tiles of an FP32C batch spread (see Deferral): work
 // items in the deferral list, folded.
 template <typename D, int DIMS>
-__global__ void __launch_bounds__(kTileThreads, 4)
+__global__ void __launch_bounds__(kDenseThreads, 2)
 batch_spread_dense_kernel(const BatchInst* __restrict__ insts, BatchTable t, const PointRec* __restrict__ recs,
                           const float4* __restrict__ forces, const int* __restrict__ off,
                           const int* __restrict__ list, const int* __restrict__ count)
@@ -276,7 +276,7 @@ batch_spread_dense_kernel(const BatchInst* __restrict__ insts, BatchTable t, con
 		copy_to_shared(&so, t.io + cur_inst);
 		__syncthreads();
 		const CompPtrs& fe = so.fe;
-		spread_tile<D, DIMS, true>(si.g, si.ts, recs, forces, off + si.bin_s, fe, cur_local, cur_comp);
+		spread_tile<D, DIMS, true, kDenseThreads>(si.g, si.ts, recs, forces, off + si.bin_s, fe, cur_local, cur_comp);
 		__syncthreads();
 	}
 }
@@ -340,7 +340,7 @@ struct Batch {
 	int bins_s = 0, bins_i = 0;
 	std::vector<int> nitem_s, nitem_i;  // work items per instance
 	long long items_s = 0, items_i = 0; // of all instances
-	size_t smem_s = 0, smem_i = 0;
+	size_t smem_s = 0, smem_d = 0, smem_i = 0;     // spread, dense FP32C spread, interpolation CTAs
 	int grid_s = 0, grid_i = 0, grid_bin = 1;
 	BatchInst* d_inst = nullptr;
 	size_t bins_cap = 0;
@@ -461,7 +461,7 @@ ibk_status batch_run_impl(Batch& b, int op, cudaStream_t s)
 			else
 				batch_spread_kernel<D, DIMS><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
 					b.d_inst, t, b.d_next, b.d_recs, b.d_forces, b.d_off, defer);
-			batch_spread_dense_kernel<D, DIMS><<<b.grid_s, kTileThreads, b.smem_s, s>>>(
+			batch_spread_dense_kernel<D, DIMS><<<std::min(b.grid_s, 2 * b.num_sms), kDenseThreads, b.smem_d, s>>>(
 				b.d_inst, t, b.d_recs, b.d_forces, b.d_off, defer.list, defer.count);
 			b.launches += 1;
 		}
@@ -503,7 +503,7 @@ ibk_status batch_prepare_impl(Batch& b)
 	};
 	if constexpr (PREC == IBK_PRECISION_FP32C) {
 		if ((st = cuda_check(cudaFuncSetAttribute(batch_spread_dense_kernel<D, DIMS>,
-		                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_s),
+		                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_d),
 		                     "cudaFuncSetAttribute")) != IBK_OK) return st;
 		st = b.config.spread_threads == 512 ? prepare_spread(batch_spread_kernel<D, DIMS, 512>, 512)
 		                                    : prepare_spread(batch_spread_kernel<D, DIMS>, kTileThreads);
@@ -634,7 +634,7 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 	std::vector<BatchInst> inst(b.count);
 	std::vector<int> nitem_s(b.count), nitem_i(b.count);
 	long long bins_s = 0, bins_i = 0, items_s = 0, items_i = 0;
-	size_t smem_max = 0, limit_max = 0, region_max = 0;
+	size_t smem_max = 0, limit_max = 0, dense_max = 0, region_max = 0;
 	for (int i = 0; i < b.count; ++i) {
 		BatchInst& bi = inst[i];
 		bi.g = b.geo[i];
@@ -661,6 +661,7 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 		if (bins_s >= (1LL << 30) || bins_i >= (1LL << 30) || items_s >= (1LL << 30) || items_i >= (1LL << 30))
 			return set_error(IBK_ERR_INVALID_ARGUMENT, "batch has too many tiles");
 		smem_max = std::max(smem_max, spread_tile_bytes(bi.g, bi.ts, b.M, b.precision));
+		dense_max = std::max(dense_max, dense_tile_bytes(bi.ts, b.dims));
 		limit_max = std::max(limit_max, spread_limit_bytes(bi.g, bi.ts, b.M, b.precision));
 		region_max = std::max(region_max, interp_region_bytes(bi.g, bi.ti, b.M));
 	}
@@ -712,6 +713,7 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 	b.items_s = items_s;
 	b.items_i = items_i;
 	b.smem_s = smem_s;
+	b.smem_d = dense_max;
 	b.smem_i = region_max;
 	b.config = cfg;
 	std::fill(b.map_ptr.begin(), b.map_ptr.end(), nullptr);   // boxes follow the tiles

@@ -92,6 +92,7 @@ constexpr int kMaxTileExtent = 64;
 // limit on tile shapes, and an interpolation CTA's staged region (largest
 // component, stencil width M), in bytes.
 size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision);
+size_t dense_tile_bytes(const TileGeom& tg, int dims);     // of a dense FP32C spread CTA
 size_t spread_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision);
 size_t interp_region_bytes(const GridGeom& g, const TileGeom& tg, int M);
 // Staged interpolation region of component c relative to a tile's first

@@ -160,15 +160,16 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 		auto kern = few ? spread_tile_kernel<D, DIMS, kFewThreads> : spread_tile_kernel<D, DIMS>;
 		const int nt = few ? kFewThreads : kTileThreads;
 		auto dense = spread_dense_kernel<D, DIMS>;
-		if ((s = set_smem(kern, smem)) != IBK_OK || (s = set_smem(dense, smem)) != IBK_OK) return s;
+		const size_t dsmem = folded_layout(tg, DIMS).bytes;
+		if ((s = set_smem(kern, smem)) != IBK_OK || (s = set_smem(dense, dsmem)) != IBK_OK) return s;
 		if ((s = launch(plan, "spread_tile_kernel", a.stream, [&] {
 			kern<<<tg.num_tiles, nt, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer);
 		})) != IBK_OK) return s;
 		// no face can receive more terms than there are points
 		if (a.n <= 2 * kFoldChunk) return IBK_OK;
-		const int gd = std::max(1, std::min(tg.num_tiles * DIMS, 4 * plan.num_sms));
+		const int gd = std::max(1, std::min(tg.num_tiles * DIMS, 2 * plan.num_sms));
 		return launch(plan, "spread_dense_kernel", a.stream, [&] {
-			dense<<<gd, kTileThreads, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer.list, b.defer.count);
+			dense<<<gd, kDenseThreads, dsmem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer.list, b.defer.count);
 		});
 	}
 }
@@ -383,6 +384,8 @@ size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int M, int preci
 {
 	return spread_smem_bytes(g, tg, M, precision);
 }
+
+size_t dense_tile_bytes(const TileGeom& tg, int dims) { return folded_layout(tg, dims).bytes; }
 
 size_t spread_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
 {

@@ -550,74 +550,101 @@ __device__ __forceinline__ void write_tile(double* __restrict__ out, const CompG
 	}
 }
 
+// Shared memory of the folded FP32C form, in words: `copies` copies of the
+// tile's accumulators, `stride` apart (8 mod 32, so that a face's copies lie
+// in different banks), then the FP64 totals; four copies where they fit.
+struct FoldedLayout {
+	int copies, stride;
+	size_t bytes;
+};
+
+__host__ __device__ inline FoldedLayout folded_layout(const TileGeom& tg, int dims)
+{
+	const int words = spread_strides(tg.T[0], tg.T[1], tg.T[2], dims).words;
+	FoldedLayout f;
+	f.stride = words + ((8 - words % 32 + 32) % 32);
+	for (f.copies = 4; f.copies >= 1; f.copies >>= 1) {
+		f.bytes = ((size_t) f.copies * f.stride + 2 * (size_t) words + 2 * kGuardWords) * 4;
+		if (f.bytes <= 200 * 1024 || f.copies == 1) break;
+	}
+	return f;
+}
+
 // The folded FP32C form of a spread tile (tiles where a face may receive
-// more terms than a 32-bit word holds): components c_lo .. c_hi - 1 one at a
-// time (the folded kernel takes one component per item), kFoldChunk
-// candidates per round, after each round the words added exactly into FP64
-// totals (integers below 2^53) and cleared.  Every thread of the CTA calls
-// it, after s_scale is set.
+// more terms than a 32-bit word holds), one component: rounds of kFoldChunk
+// candidates per copy of the accumulators, after each round the words added
+// exactly into FP64 totals (integers below 2^53) and cleared.  Neighbouring
+// lanes add to different copies: a warp's candidates crowd together in such
+// a tile, and their reductions into one copy meet in the same words.  The
+// spread of 416,000 points on 30^3 cells takes 398 us with one copy, 341 with
+// two, 306 with four and 297 with eight; 24 instances' step 1226 with one, 1253,
+// 1211 and 1302.  Every thread of the CTA calls it.
 template <typename D, int DIMS, int NT>
 __device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const TileGeom& tg,
                                                 const PointRec* __restrict__ recs, const float4* __restrict__ forces,
                                                 const RangeTable& rt, int ncand, const int* lo,
                                                 const int* cells, const bool* wrap, bool wrap_any,
-                                                unsigned acc_addr, const CompPtrs& fe,
-                                                const float* s_scale, int c_lo, int c_hi)
+                                                unsigned acc_addr, const CompPtrs& fe, float sc, int c)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	const SpreadStrides ss = spread_strides(tg.T[0], tg.T[1], DIMS == 3 ? tg.T[2] : 1, DIMS);
+	const FoldedLayout fl = folded_layout(tg, DIMS);
 	int* words = reinterpret_cast<int*>(smem_raw + 4 * kGuardWords);
-	double* total = reinterpret_cast<double*>(words + ss.words);     // ss.words is a multiple of 4
-	for (int c = c_lo; c < c_hi; ++c) {
-		const CompGeom& cg = g.comp[c];
-		int e[3] = {1, 1, 1};
+	double* total = reinterpret_cast<double*>(words + fl.copies * fl.stride);     // the stride is a multiple of 4
+	const unsigned mine = acc_addr + 4u * (unsigned) ((threadIdx.x & (fl.copies - 1)) * fl.stride);
+	const CompGeom& cg = g.comp[c];
+	int e[3] = {1, 1, 1};
 #pragma unroll
-		for (int d = 0; d < DIMS; ++d) e[d] = min(tg.T[d], cg.points[d] - lo[d]);
-		for (int i = threadIdx.x; i < ss.words; i += NT) { words[i] = 0; total[i] = 0.0; }
-		__syncthreads();
-		const float sc = s_scale[c];
-		if (sc != 0.0f) {
-			int r = 0;
-			for (int chunk = 0; chunk < ncand; chunk += kFoldChunk) {
-				for (int it = chunk + threadIdx.x; it < min(ncand, chunk + kFoldChunk); it += NT) {
-					const int slot = range_walk(rt, r, it);
-					const PointRec rec = load_rec(recs + slot);
-					const int sft = rt.shift[r];
-					int l[DIMS];
-					float dl[DIMS];
+	for (int d = 0; d < DIMS; ++d) e[d] = min(tg.T[d], cg.points[d] - lo[d]);
+	for (int i = threadIdx.x; i < fl.copies * fl.stride; i += NT) words[i] = 0;
+	for (int i = threadIdx.x; i < ss.words; i += NT) total[i] = 0.0;
+	__syncthreads();
+	if (sc != 0.0f) {
+		const int round = kFoldChunk * fl.copies;      // a copy's share: the candidates of its residue
+		int r = 0;
+		for (int chunk = 0; chunk < ncand; chunk += round) {
+			for (int it = chunk + threadIdx.x; it < min(ncand, chunk + round); it += NT) {
+				const int slot = range_walk(rt, r, it);
+				const PointRec rec = load_rec(recs + slot);
+				const int sft = rt.shift[r];
+				int l[DIMS];
+				float dl[DIMS];
 #pragma unroll
-					for (int d = 0; d < DIMS; ++d) {
-						const bool own = tg.tag_mac && d == c;
-						l[d] = rec_origin(rec.org, d) + unpack8(sft, d) + (own ? rec_own_shift(rec.org, d) : 0);
-						dl[d] = own ? rec.dn[d] : rec.dh[d];
-					}
-					const float f = __ldg(reinterpret_cast<const float*>(forces + slot) + c) * sc;
-					if (!wrap_any) {
-						spread_fix<D, DIMS>(acc_addr, l, dl, f, e, ss.S1, ss.S2);
-					} else {
-						float w[DIMS][D::M];
-#pragma unroll
-						for (int d = 0; d < DIMS; ++d) weights32<D>(dl[d], w[d]);
-						spread_wrapped<D, DIMS>(l, e, cells, wrap, ss.S1, ss.S2,
-							[&](int li, int v) { red_shared(acc_addr + 4u * (unsigned) li, v); },
-							[&](int m0, int m1, int m2) {
-								const float w12 = DIMS == 3 ? w[1][m1] * w[2][m2] : w[1][m1];
-								return fix_term(w[0][m0] * f, w12);
-							});
-					}
+				for (int d = 0; d < DIMS; ++d) {
+					const bool own = tg.tag_mac && d == c;
+					l[d] = rec_origin(rec.org, d) + unpack8(sft, d) + (own ? rec_own_shift(rec.org, d) : 0);
+					dl[d] = own ? rec.dn[d] : rec.dh[d];
 				}
-				__syncthreads();
-				for (int i = threadIdx.x; i < ss.words; i += NT) {
-					total[i] += (double) words[i];
-					words[i] = 0;
+				const float f = __ldg(reinterpret_cast<const float*>(forces + slot) + c) * sc;
+				if (!wrap_any) {
+					spread_fix<D, DIMS>(mine, l, dl, f, e, ss.S1, ss.S2);
+				} else {
+					float w[DIMS][D::M];
+#pragma unroll
+					for (int d = 0; d < DIMS; ++d) weights32<D>(dl[d], w[d]);
+					spread_wrapped<D, DIMS>(l, e, cells, wrap, ss.S1, ss.S2,
+						[&](int li, int v) { red_shared(mine + 4u * (unsigned) li, v); },
+						[&](int m0, int m1, int m2) {
+							const float w12 = DIMS == 3 ? w[1][m1] * w[2][m2] : w[1][m1];
+							return fix_term(w[0][m0] * f, w12);
+						});
 				}
-				__syncthreads();
 			}
+			__syncthreads();
+			for (int i = threadIdx.x; i < ss.words; i += NT) {
+				double t = total[i];
+				for (int k = 0; k < fl.copies; ++k) {
+					t += (double) words[k * fl.stride + i];
+					words[k * fl.stride + i] = 0;
+				}
+				total[i] = t;
+			}
+			__syncthreads();
 		}
-		const double inv = sc != 0.0f ? 1.0 / (double) sc : 0.0;
-		write_tile<DIMS, NT>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [&](int li) { return total[li] * inv; });
-		__syncthreads();
 	}
+	const double inv = sc != 0.0f ? 1.0 / (double) sc : 0.0;
+	write_tile<DIMS, NT>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [&](int li) { return total[li] * inv; });
+	__syncthreads();
 }
 
 // One FP32C spread tile; every thread of the CTA calls it.  FOLDED takes one
@@ -678,8 +705,9 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 	force_maxima<NT>(rt, ncand, forces, s_fmax);
 	if constexpr (FOLDED) {
 		if (threadIdx.x < kMaxDims) s_scale[threadIdx.x] = fix_scale(s_fmax[threadIdx.x], max_weight<D, DIMS>(), kFoldChunk);
-		spread_tile_folded<D, DIMS, NT>(g, tg, recs, forces, rt, ncand, lo, cells, wrap, wrap_any, acc_addr,
-		                                fe, s_scale, c_lo, c_hi);
+		__syncthreads();
+		spread_tile_folded<D, DIMS, NT>(g, tg, recs, forces, rt, ncand, lo, cells, wrap, wrap_any, acc_addr, fe, s_scale[comp],
+		                                comp);
 		return;
 	}
 	// one pass unless a face may receive more than 2 kFoldChunk terms (the
@@ -1116,8 +1144,7 @@ __device__ __forceinline__ void spread_any64(const GridGeom& g, const TileGeom& 
 }
 
 // Shared memory of a spread CTA.  FP32C: every component's accumulator words
-// (4 bytes per face; the folded form's words and totals of one component, or
-// the occupancy grid, where larger) between guard words.
+// (4 bytes per face; the occupancy grid where larger) between guard words.
 __host__ __device__ inline size_t spread_smem_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
 {
 	if (precision != IBK_PRECISION_FP32C) return spread64_smem_bytes(g, tg, M);
@@ -1157,8 +1184,10 @@ spread_tile64_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ 
 // The deferred dense tiles of an FP32C spread, folded (see Deferral); the
 // grid strides over the list, whose length the one-pass kernel left on the
 // device.
+constexpr int kDenseThreads = 512;
+
 template <typename D, int DIMS>
-__global__ void __launch_bounds__(kTileThreads, 4)
+__global__ void __launch_bounds__(kDenseThreads, 2)
 spread_dense_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, const float4* __restrict__ forces,
                     const int* __restrict__ off, CompPtrs fe, const int* __restrict__ list,
                     const int* __restrict__ count)
@@ -1166,7 +1195,7 @@ spread_dense_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, 
 	const int m = *count;
 	for (int k = blockIdx.x; k < m; k += gridDim.x) {
 		const int v = __ldg(list + k);
-		spread_tile<D, DIMS, true>(g, tg, recs, forces, off, fe, v >> 2, v & 3);
+		spread_tile<D, DIMS, true, kDenseThreads>(g, tg, recs, forces, off, fe, v >> 2, v & 3);
 		__syncthreads();
 	}
 }
