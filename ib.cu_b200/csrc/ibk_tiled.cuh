@@ -552,7 +552,8 @@ __device__ __forceinline__ void write_tile(double* __restrict__ out, const CompG
 
 // Shared memory of the folded FP32C form, in words: `copies` copies of the
 // tile's accumulators, `stride` apart (8 mod 32, so that a face's copies lie
-// in different banks), then the FP64 totals; four copies where they fit.
+// in different banks), then the FP64 totals; up to eight copies while two CTAs
+// fit on an SM (four at 16^3 tiles, eight at 8^3).
 struct FoldedLayout {
 	int copies, stride;
 	size_t bytes;
@@ -563,9 +564,9 @@ __host__ __device__ inline FoldedLayout folded_layout(const TileGeom& tg, int di
 	const int words = spread_strides(tg.T[0], tg.T[1], tg.T[2], dims).words;
 	FoldedLayout f;
 	f.stride = words + ((8 - words % 32 + 32) % 32);
-	for (f.copies = 4; f.copies >= 1; f.copies >>= 1) {
+	for (f.copies = 8; f.copies >= 1; f.copies >>= 1) {
 		f.bytes = ((size_t) f.copies * f.stride + 2 * (size_t) words + 2 * kGuardWords) * 4;
-		if (f.bytes <= 200 * 1024 || f.copies == 1) break;
+		if (f.bytes <= (f.copies > 2 ? 112 : 200) * 1024 || f.copies == 1) break;
 	}
 	return f;
 }
@@ -577,8 +578,8 @@ __host__ __device__ inline FoldedLayout folded_layout(const TileGeom& tg, int di
 // lanes add to different copies: a warp's candidates crowd together in such
 // a tile, and their reductions into one copy meet in the same words.  The
 // spread of 416,000 points on 30^3 cells takes 398 us with one copy, 341 with
-// two, 306 with four and 297 with eight; 24 instances' step 1226 with one, 1253,
-// 1211 and 1302.  Every thread of the CTA calls it.
+// two, 306 with four and 297 with eight; 24 instances 1226, 1253, 1211 and 1302
+// us with the same number in every tile, 1193 with this rule.  Every thread of the CTA calls it.
 template <typename D, int DIMS, int NT>
 __device__ __forceinline__ void spread_tile_folded(const GridGeom& g, const TileGeom& tg,
                                                 const PointRec* __restrict__ recs, const float4* __restrict__ forces,
