@@ -572,7 +572,7 @@ constexpr int kMaxRun = 64;
 // half the update and the direction as passes of their own: 336 + 237 + 241
 // us).  At most three CTAs per SM: with four (64 registers) it spills, 2 to 5 %
 // slower.
-constexpr int kDirX = 64, kDirY = 8, kDirRows = 2, kDirThreads = 256, kDirBlocks = 3;
+constexpr int kDirX = 64, kDirY = 16, kDirRows = 4, kDirThreads = 256, kDirBlocks = 2;
 constexpr int kDirStride = kDirX + 2;
 
 __global__ void __launch_bounds__(kDirThreads, kDirBlocks)
@@ -720,7 +720,7 @@ struct PolyTile {
 // tile's; the small one has three times the blocks.  512 x 256 x 512 faces
 // 20.2 ms a solve against 23.4 ms, 256 x 128 x 256 3.43 against 3.57, 128^3
 // 1.11 against 1.09, 117 x 234 x 117 1.85 against 1.76, 64^3 0.49 against 0.46.
-using PolyWide = PolyTile<64, 8, 3, 1>;
+using PolyWide = PolyTile<64, 8, 4, 1>;
 using PolySmall = PolyTile<32, 16, 1, 2>;
 
 struct ChebWeights { double w[4]; };
