@@ -558,20 +558,20 @@ __device__ __forceinline__ void fill_table(const FluidOps& o, int axis, int firs
 		t[i] = axis_coef(o.ax[axis], axis < o.dims, o.lambda, fold_index(o.ax[axis], first + i));
 }
 
-// Time of one step of polynomial_kernel's wide tile over the small tile's
-// (from the solves timed above).
+// Time of one step of polynomial_kernel's wide tile over the small tile's, from
+// the solves timed above; it puts the line a little below 128^3 faces.
 constexpr double kWideStep = 1.5;
 
 // Longest run of planes per block (bounds the tables along z).
 constexpr int kMaxRun = 64;
 
-// direction_apply_kernel's tile: 64 x 8 columns, 256 threads with two
-// neighbouring rows each; the first 144 threads also hold one column each of
+// direction_apply_kernel's tile: 64 x 16 columns, 256 threads with four
+// neighbouring rows each; the first 160 threads also hold one column each of
 // the halo.  Bound by HBM: 48 bytes per face, the next plane's z, d and x
-// loaded a plane ahead.  512 x 256 x 512 faces: 551 us, 5.85 TB/s (operator,
+// loaded a plane ahead.  512 x 256 x 512 faces: 511 us, 6.3 TB/s (operator,
 // half the update and the direction as passes of their own: 336 + 237 + 241
-// us).  At most three CTAs per SM: with four (64 registers) it spills, 2 to 5 %
-// slower.
+// us; 64 x 8 columns with two rows a thread, three CTAs per SM: 551 us, and 2
+// to 5 % more with four CTAs, which spill).
 constexpr int kDirX = 64, kDirY = 16, kDirRows = 4, kDirThreads = 256, kDirBlocks = 2;
 constexpr int kDirStride = kDirX + 2;
 
@@ -708,7 +708,12 @@ direction_apply_kernel(FluidOps o, double* __restrict__ sc, const double* __rest
 // step's plane p - 1, the second's p - 2 and the third's p - 3, each from the
 // part that was formed as soon as the planes below were there: what follows
 // the barrier is three independent parts.  Columns and planes at the rim of
-// the halo hold values that nothing inside uses.
+// the halo hold values that nothing inside uses.  512 x 256 x 512 faces: 687 us
+// (the three steps and half the update as passes of their own: 450 + 2 x 473 +
+// 237 us), against 330 us for its 32 bytes per face: what bounds it is the
+// shared-memory pipe (about 60 % of its peak: 11 64-bit accesses per column
+// and plane) and FP64 issue (26 %) taking turns between barriers, at one CTA of
+// 128 registers per thread.
 template <int EX_, int TY_, int ROWS_, int BLOCKS_>
 struct PolyTile {
 	static constexpr int EX = EX_, TY = TY_, ROWS = ROWS_, BLOCKS = BLOCKS_, HALO = 3;
@@ -716,10 +721,11 @@ struct PolyTile {
 	static constexpr int PLANE = EX * EY, BYTES = 6 * PLANE * (int) sizeof(double);
 	static_assert(THREADS % 32 == 0, "whole warps");
 };
-// Two thirds of the wide tile's columns are the block's own, half of the small
-// tile's; the small one has three times the blocks.  512 x 256 x 512 faces
-// 20.2 ms a solve against 23.4 ms, 256 x 128 x 256 3.43 against 3.57, 128^3
-// 1.11 against 1.09, 117 x 234 x 117 1.85 against 1.76, 64^3 0.49 against 0.46.
+// Of the wide tile's columns 74 % are the block's own, of the small tile's
+// half; the small one has four times the blocks.  With three rows a thread in
+// the wide tile (743 us): 512 x 256 x 512 faces 20.2 ms a solve against 23.4
+// ms, 256 x 128 x 256 3.43 against 3.57, 128^3 1.11 against 1.09, 117 x 234 x
+// 117 1.85 against 1.76, 64^3 0.49 against 0.46.
 using PolyWide = PolyTile<64, 8, 4, 1>;
 using PolySmall = PolyTile<32, 16, 1, 2>;
 
