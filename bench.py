@@ -899,10 +899,10 @@ def run_fluid(ibk, W, dev, steps, warmup=1, workload="large-channel"):
         del out
     ms = float(np.median(times))
     iters = int(np.median(its))
-    # Chebyshev-preconditioned iteration, bytes per face: operator (d in, q
-    # out: 16), x / r update (48), the three polynomial steps (16 + 24 + 24),
-    # direction (24)
-    per_iter_bytes = 152.0 * d.size
+    # Chebyshev-preconditioned iteration, bytes per face: direction, x and
+    # operator in one kernel (z, d, x in; d, x, q out: 48), residual and
+    # polynomial in another (r, q in; r, z out: 32)
+    per_iter_bytes = 80.0 * d.size
     peak, _ = measured_peaks()
     res = {"faces": d.size, "grid": "x".join(str(int(round(l / 0.025))) for l in w.lengths) + " (x faces)",
            "steps": steps, "ms_per_step": ms,
@@ -910,7 +910,7 @@ def run_fluid(ibk, W, dev, steps, warmup=1, workload="large-channel"):
            "iteration_gbs": per_iter_bytes * iters / (ms * 1e-3) / 1e9,
            "iteration_frac_of_hbm": per_iter_bytes * iters / (ms * 1e-3) / 1e9 / peak,
            "note": "FP64 matrix-free operator and PCG with the reference's degree-4 Chebyshev preconditioner "
-                   "(Gershgorin interval), the convergence test read back once per iteration; median of the "
+                   "(Gershgorin interval), the convergence test on the device; median of the "
                    "timed steps, CUDA events"}
     del d, plan, u, f, rhs
     torch.cuda.empty_cache()
