@@ -275,14 +275,19 @@ ibk_status ibk_plan_create(const ibk_domain* domain, int tag, int refinement, ib
 	const GridGeom& g = plan->g;
 	const ibk_grid_info& info = plan->info;
 	// both operators on the default tiles (16^3 cells, smaller on small
-	// grids), so one binning serves a spread and an interpolation.  FP64 tiles
-	// get small earlier (eight instead of four per axis): a tile's candidates
-	// are a serial chain there, and a 64^3 grid of 16^3 tiles has 64 of them
-	// (one red cell on it, both operators: 95 -> 81 us).
-	int small[kMaxDims];
-	for (int d = 0; d < dims; ++d) small[d] = std::min(16, std::max(8, g.comp[0].cells[d] / 8));
-	const bool early = precision == IBK_PRECISION_FP64 && dims == 3;
-	plan->tiles = make_tiles(g, tag, info.meshwidths, early ? small : nullptr);
+	// grids), so one binning serves a spread and an interpolation.  Where those
+	// are fewer than the SMs, FP64 plans take smaller ones (eight instead of
+	// four per axis): a tile's candidates are a serial chain there (one red cell
+	// on 64^3, 64 tiles of 16^3, both operators: 95 -> 81 us).  Not where x would
+	// get an odd extent, whose regions the interpolation cannot stage by TMA
+	// (110 x 110 x 220 cells in tiles of 13: 143 instead of 105 us).
+	plan->tiles = make_tiles(g, tag, info.meshwidths);
+	if (precision == IBK_PRECISION_FP64 && dims == 3 && plan->tiles.num_tiles <= plan->num_sms) {
+		int small[kMaxDims];
+		for (int d = 0; d < dims; ++d) small[d] = std::min(16, std::max(8, g.comp[0].cells[d] / 8));
+		const TileGeom t = make_tiles(g, tag, info.meshwidths, small);
+		if (t.T[0] % 2 == 0) plan->tiles = t;
+	}
 	plan->spread_tiles = plan->tiles;
 	plan->tag = tag;
 	for (int d = 0; d < dims; ++d)
