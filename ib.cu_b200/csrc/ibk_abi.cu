@@ -168,8 +168,9 @@ ibk_status ensure_scratch(Plan& plan, int slot, size_t bytes, cudaStream_t strea
 		return set_error(IBK_ERR_OUT_OF_MEMORY, "cudaMalloc of plan scratch failed");
 	}
 	if (zero) {
-		e = cudaMemset(p, 0, want);
-		if (e != cudaSuccess) { cudaFree(p); return set_error(IBK_ERR_CUDA, std::string("cudaMemset: ") + cudaGetErrorString(e)); }
+		// on the caller's stream: a non-blocking one does not wait for the default stream
+		e = cudaMemsetAsync(p, 0, want, stream);
+		if (e != cudaSuccess) { cudaFree(p); return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e)); }
 	}
 	s.ptr = p;
 	s.bytes = want;
