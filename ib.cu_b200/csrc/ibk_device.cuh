@@ -221,11 +221,13 @@ static __device__ __noinline__ double bspline3_recursion(double r) { return Bspl
 // product with 0 or 1 and a sum with 0 are exact); 19 FP64 operations a
 // weight instead of about 60.  Closer to 0 than 2^-50 the recursion's own
 // roundings of delta +- 1/2 let both neighbouring indicators (or neither) be
-// 1, so there it is evaluated as it stands; 0 itself is regular.
+// 1, so there it is evaluated as it stands; 0 itself is regular.  So it is
+// outside [-1, 0]: positions beyond the range of an index saturate it, and a
+// point that far away has weights of 0 (or NaN).
 template <>
 __device__ __forceinline__ void weights64<Delta<kBspline, 3>>(double delta, double* w)
 {
-	if (!(delta <= -0x1p-50 || delta == 0.0)) {
+	if (!((delta >= -1.0 && delta <= -0x1p-50) || delta == 0.0)) {
 		w[0] = bspline3_recursion(__dadd_rn(delta, -1.0));
 		w[1] = bspline3_recursion(__dadd_rn(delta, 0.0));
 		w[2] = bspline3_recursion(__dadd_rn(delta, 1.0));

@@ -71,3 +71,28 @@ def test_points_on_and_next_to_nodes(ibk, oracle, cuda):
     far = np.concatenate([rng.choice([-1.0, 1.0], 500) * 10.0 ** rng.uniform(-320, 7, 500) for _ in range(3)])
     for c, got in enumerate(device_keys(plan, far, cuda)):
         assert np.array_equal(got, oracle.sort_keys(g, c, far))
+
+
+@pytest.mark.parametrize("tiles", [None, (16, 16, 16)])
+def test_positions_beyond_the_index_range(ibk, oracle, cuda, tiles):
+    """Positions more than 2^31 cells past a wall, where the stencil's index
+    saturates: the delta function is 0 there, so they leave the grid as it is
+    and take no velocity."""
+    rng = np.random.default_rng(12)
+    L, solid, n, far = [1.6, 1.6, 1.6], [0, 1, 0], 300, 40
+    g = oracle.geometry(3, L, solid, oracle.TAG_MAC, 64)
+    plan = plan_for(ibk, 3, L, solid, 0, 64, 0, 3)
+    if tiles is not None:
+        plan.set_tiles(tiles, tiles)
+    near = [rng.uniform(0, l, n) for l in L]
+    f = [rng.normal(size=n) for _ in range(3)]
+    away = [rng.uniform(0, 1.6, far), 10.0 ** rng.uniform(8, 25, far) * rng.choice([-1, 1], far), rng.uniform(0, 1.6, far)]
+    x = np.concatenate([np.concatenate([a, b]) for a, b in zip(near, away)])
+    fl = np.concatenate([np.concatenate([a, rng.normal(size=far)]) for a in f])
+    want_fe, fa = oracle.spread(g, np.concatenate(near), np.concatenate(f), with_abs=True)
+    check_spread(device_spread(plan, x, fl, cuda), want_fe, fa)
+    ue = [rng.normal(size=int(g.size[c])) for c in range(3)]
+    ul = device_interp(plan, x, ue, cuda).reshape(3, n + far)
+    assert np.array_equal(ul[:, n:], np.zeros((3, far)))
+    want, ua = oracle.interpolate(g, np.concatenate(near), ue, with_abs=True)
+    check_interp(np.ascontiguousarray(ul[:, :n]).reshape(-1), want, ua)
