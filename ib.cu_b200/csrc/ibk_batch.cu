@@ -495,24 +495,20 @@ ibk_status batch_prepare_impl(Batch& b)
 	int occ_s = 0, occ_i = 0;
 	// the spread kernel's shared memory and resident CTAs
 	auto prepare_spread = [&](auto ks, int nts) -> ibk_status {
-		ibk_status ps = cuda_check(cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_s),
-		                           "cudaFuncSetAttribute");
+		const ibk_status ps = allow_smem(ks);
 		if (ps != IBK_OK) return ps;
 		return cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks, nts, b.smem_s),
 		                  "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
 	};
 	if constexpr (PREC == IBK_PRECISION_FP32C) {
-		if ((st = cuda_check(cudaFuncSetAttribute(batch_spread_dense_kernel<D, DIMS>,
-		                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_d),
-		                     "cudaFuncSetAttribute")) != IBK_OK) return st;
+		if ((st = allow_smem(batch_spread_dense_kernel<D, DIMS>)) != IBK_OK) return st;
 		st = b.config.spread_threads == 512 ? prepare_spread(batch_spread_kernel<D, DIMS, 512>, 512)
 		                                    : prepare_spread(batch_spread_kernel<D, DIMS>, kTileThreads);
 	} else {
 		st = prepare_spread(batch_spread64_kernel<D, DIMS>, s64_threads<DIMS>());
 	}
 	if (st != IBK_OK) return st;
-	if ((st = cuda_check(cudaFuncSetAttribute(ki, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) b.smem_i),
-	                     "cudaFuncSetAttribute")) != IBK_OK) return st;
+	if ((st = allow_smem(ki)) != IBK_OK) return st;
 	if ((st = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_i, ki, kTileThreads, b.smem_i),
 	                     "cudaOccupancyMaxActiveBlocksPerMultiprocessor")) != IBK_OK) return st;
 	if (occ_s < 1 || occ_i < 1) return set_error(IBK_ERR_UNSUPPORTED, "batch tiles need more shared memory than an SM has");

@@ -127,4 +127,21 @@ bool grid_tensor_map(CUtensorMap* map, const double* base, const CompGeom& cg, i
 ibk_status set_error(ibk_status s, const std::string& msg);
 ibk_status check_launch(const char* what);
 
+// The most dynamic shared memory that any launch takes: tile shapes are held
+// to 200 KB, beside which an FP64 spread stages up to 10.5 KB of weights; with
+// the kernels' static shared memory it stays below the 227 KB of a CTA.
+constexpr int kMaxDynamicSmem = 216 * 1024;
+
+// Opt the kernel in to that much (static shared memory counts against the 48
+// KB default too, so every tile kernel needs it).  The limit belongs to the
+// kernel, not to the launch: always the same value, so that no thread or
+// batch lowers it under another's launch.
+template <typename K>
+ibk_status allow_smem(K kernel)
+{
+	const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+	return IBK_OK;
+}
+
 } // namespace ibk

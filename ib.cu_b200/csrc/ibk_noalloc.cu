@@ -142,8 +142,7 @@ ibk_status run(const GridGeom& g, int tag, int n, const double* x, ConstCompPtrs
 	if ((s = check_launch("bin_scatter_kernel")) != IBK_OK) return s;
 	const size_t smem = interp_smem_bytes<M>(g, tg);
 	auto kern = interp_tile_kernel<D, DIMS, PREC>;
-	e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+	if ((s = allow_smem(kern)) != IBK_OK) return s;
 	// regions are staged with plain loads here (use_tma = 0), so the kernel
 	// has no device-side check to report and gets no status word
 	TmaMaps maps{};

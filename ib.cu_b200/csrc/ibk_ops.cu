@@ -48,16 +48,6 @@ ibk_status interp_direct(Plan& plan, const OpArgs& a, ConstCompPtrs ue, double* 
 	});
 }
 
-// Opt the kernel in to `bytes` of dynamic shared memory (static shared
-// memory counts against the 48 KB default too, so this is always set).
-template <typename K>
-ibk_status set_smem(K kernel, size_t bytes)
-{
-	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
-	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-	return IBK_OK;
-}
-
 // What the binning leaves: records in bin order, the bin offsets and, for an
 // FP32C spread, the points' forces beside the records and the deferral list
 // with its count zeroed.
@@ -107,7 +97,7 @@ ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, Binned& o
 	if (a.n <= (tail ? kSmallThreads : kSmallPoints) && tg.num_bins <= kSmallBins) {
 		const size_t smem = sizeof(int) * (size_t) tg.num_bins;
 		auto kern = bin_small_kernel<M, DIMS>;
-		if ((s = set_smem(kern, smem)) != IBK_OK) return s;
+		if ((s = allow_smem(kern)) != IBK_OK) return s;
 		return launch(plan, "bin_small_kernel", a.stream, [&] {
 			kern<<<1, kSmallThreads, smem, a.stream>>>(g, tg, a.n, a.x, off, recs, bf, clear);
 		});
@@ -138,7 +128,7 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 	ibk_status s;
 	if constexpr (PREC == IBK_PRECISION_FP64) {
 		auto kern = spread_tile64_kernel<D, DIMS>;
-		if ((s = set_smem(kern, smem)) != IBK_OK) return s;
+		if ((s = allow_smem(kern)) != IBK_OK) return s;
 		// Few tiles with many candidates each (about 2.5 per point): several
 		// CTAs share a tile's candidates and add their sums to zeroed faces.
 		const long long items = (long long) tg.num_tiles * DIMS, cand = 5LL * a.n / (2 * tg.num_tiles);
@@ -161,7 +151,7 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 		const int nt = few ? kFewThreads : kTileThreads;
 		auto dense = spread_dense_kernel<D, DIMS>;
 		const size_t dsmem = folded_layout(tg, DIMS).bytes;
-		if ((s = set_smem(kern, smem)) != IBK_OK || (s = set_smem(dense, dsmem)) != IBK_OK) return s;
+		if ((s = allow_smem(kern)) != IBK_OK || (s = allow_smem(dense)) != IBK_OK) return s;
 		if ((s = launch(plan, "spread_tile_kernel", a.stream, [&] {
 			kern<<<tg.num_tiles, nt, smem, a.stream>>>(*a.g, tg, b.recs, b.forces, b.off, fe, b.defer);
 		})) != IBK_OK) return s;
@@ -252,7 +242,7 @@ ibk_status launch_interp(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 		use_tma = grid_tensor_map(&maps.map[c], ue.p[c], g.comp[c], DIMS, box);
 	}
 	auto kern = interp_tile_kernel<D, DIMS, PREC>;
-	ibk_status s = set_smem(kern, smem);
+	ibk_status s = allow_smem(kern);
 	if (s != IBK_OK) return s;
 	return launch(plan, "interp_tile_kernel", a.stream, [&] {
 		kern<<<dim3(tg.num_tiles, DIMS), kTileThreads, smem, a.stream>>>(g, tg, a.n, a.x, b.recs, b.off, ue, ul,

@@ -315,3 +315,26 @@ def test_ensemble_instances_against_oracle(ibk, oracle, cuda):
                     ref = want_ul[c * n:(c + 1) * n]
                     assert np.abs(got_ul[c * n:(c + 1) * n] - ref).max() <= FP32C_TOL * np.abs(ref).max(), (i, c)
         del batch, io
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_smaller_batch_leaves_the_larger_one_its_shared_memory(ibk, cuda, precision):
+    """The limit on a kernel's shared memory is the process's: a batch of
+    small tiles set up later must not lower it for one of large tiles."""
+    import torch
+    from ib_cu_b200 import workloads as W
+    rng = np.random.default_rng(9)
+    batches = []
+    for side in (64, 32):
+        w = W.small_instance(rng, side, 2, False, f"side{side}")
+        case = Case(ibk, w, precision, cuda, side)
+        batches.append((case, ibk.Batch([ibk.Instance(ibk.Mac(w.refinement), _domain(ibk, w))], ibk.Bspline(3), precision,
+                                        max_points=w.n)))
+    case, batch = batches[0]
+    batch.bind([case.io()])
+    batch.run(ibk.OP_SPREAD)
+    batch.run(ibk.OP_INTERPOLATE)
+    torch.cuda.synchronize()
+    assert np.array_equal(case.ul.cpu().numpy(), case.plan_interp())
+    for got, want in zip(case.fe, case.plan_spread()):
+        assert np.abs(got.cpu().numpy() - want).max() <= FP64_SPREAD_TOL * np.abs(want).max()
