@@ -82,8 +82,14 @@ ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, Binned& o
 	const int nb = blocks_for(a.n, 256);
 	BinForces bf{f, g.res, nullptr};
 	int* clear = nullptr;
+	// Room for as many forces as records, from the first spread on: a spread
+	// under capture then finds it whenever the records' own room suffices.  An
+	// interpolation does without.
+	if (f || plan.scratch[kSlotForces].ptr) {
+		const size_t held = plan.scratch[kSlotRecs].bytes / sizeof(PointRec);
+		if ((s = ensure_scratch(plan, kSlotForces, sizeof(float4) * held, a.stream)) != IBK_OK && f) return s;
+	}
 	if (f) {
-		if ((s = ensure_scratch(plan, kSlotForces, sizeof(float4) * (size_t) need, a.stream)) != IBK_OK) return s;
 		if ((s = ensure_scratch(plan, kSlotDefer, sizeof(int) * ((size_t) tg.num_tiles * DIMS + 4), a.stream)) != IBK_OK)
 			return s;
 		bf.out = static_cast<float4*>(plan.scratch[kSlotForces].ptr);

@@ -38,3 +38,29 @@ def test_first_call_on_a_side_stream(ibk, oracle, cuda, cells, n):
     want, ua = oracle.interpolate(g, x, ue, with_abs=True)
     check_spread([t.cpu().numpy() for t in fe], want_fe, fa)
     check_interp(ul.cpu().numpy(), want, ua)
+
+
+@pytest.mark.parametrize("first", ["spread", "interpolate"])
+def test_captured_spread_takes_the_points_of_any_call_before(ibk, cuda, first):
+    """Scratch grown by an interpolation of many points also serves a captured
+    FP32C spread of as many, when spreads have only had a few points so far."""
+    import torch
+    rng = np.random.default_rng(2)
+    n, few, L = 5000, 100, [1.6, 1.6, 1.6]
+    plan = plan_for(ibk, 3, L, [0, 0, 0], 0, 64, 0, 3, ibk.FP32C)
+    x, f = (dev(a, cuda) for a in (rng.uniform(0, 1.6, 3 * n), rng.normal(size=3 * n)))
+    xs, fs = (dev(a, cuda) for a in (rng.uniform(0, 1.6, 3 * few), rng.normal(size=3 * few)))
+    ue = [dev(rng.normal(size=s), cuda) for s in plan.sizes()]
+    ul = torch.empty_like(x)
+    fe, want = ([torch.zeros(s, dtype=torch.float64, device=cuda) for s in plan.sizes()] for _ in range(2))
+    calls = [lambda: plan.spread(few, xs, fs, fe), lambda: plan.interpolate(n, x, ue, ul)]
+    for call in calls if first == "spread" else calls[::-1]:
+        call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.spread(n, x, f, fe)
+    graph.replay()
+    plan_for(ibk, 3, L, [0, 0, 0], 0, 64, 0, 3, ibk.FP32C).spread(n, x, f, want)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(fe, want))
