@@ -225,8 +225,8 @@ batch_spread_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __re
 }
 
 // Persistent FP64 spread over the active instances' (tile, component) items.
-template <typename D, int DIMS>
-__global__ void __launch_bounds__(s64_threads<DIMS>(), 4)
+template <typename D, int DIMS, bool OWNERS = s64_owners<D, DIMS>()>
+__global__ void __launch_bounds__(s64_threads<OWNERS>(), s64_ctas<OWNERS>())
 batch_spread64_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __restrict__ next,
                       const PointRec* __restrict__ recs, const int* __restrict__ off, int step)
 {
@@ -243,7 +243,7 @@ batch_spread64_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __
 		copy_to_shared(&so, t.io + inst);
 		__syncthreads();
 		const CompPtrs& fe = so.fe;
-		spread_any64<D, DIMS>(si.g, si.ts, so.n, step ? so.xn : so.x, step ? so.fs : so.fl, recs, so.pbase,
+		spread_any64<D, DIMS, OWNERS>(si.g, si.ts, so.n, step ? so.xn : so.x, step ? so.fs : so.fl, recs, so.pbase,
 		                      off + si.bin_s, fe, local / DIMS, local % DIMS);
 		__syncthreads();
 	}
@@ -451,7 +451,7 @@ ibk_status batch_run_impl(Batch& b, int op, cudaStream_t s)
 	auto spread = [&]() -> ibk_status {
 		b.launches += 1;
 		if constexpr (PREC == IBK_PRECISION_FP64) {
-			batch_spread64_kernel<D, DIMS><<<b.grid_s, s64_threads<DIMS>(), b.smem_s, s>>>(
+			batch_spread64_kernel<D, DIMS><<<b.grid_s, s64_threads<s64_owners<D, DIMS>()>(), b.smem_s, s>>>(
 				b.d_inst, t, b.d_next, b.d_recs, b.d_off, step ? 1 : 0);
 		} else {
 			Deferral defer{b.d_defer + 4, b.d_defer};
@@ -505,7 +505,7 @@ ibk_status batch_prepare_impl(Batch& b)
 		st = b.config.spread_threads == 512 ? prepare_spread(batch_spread_kernel<D, DIMS, 512>, 512)
 		                                    : prepare_spread(batch_spread_kernel<D, DIMS>, kTileThreads);
 	} else {
-		st = prepare_spread(batch_spread64_kernel<D, DIMS>, s64_threads<DIMS>());
+		st = prepare_spread(batch_spread64_kernel<D, DIMS>, s64_threads<s64_owners<D, DIMS>()>());
 	}
 	if (st != IBK_OK) return st;
 	if ((st = allow_smem(ki)) != IBK_OK) return st;
@@ -656,7 +656,7 @@ ibk_status configure(Batch& b, const ibk_batch_config& cfg)
 		items_i += nitem_i[i];
 		if (bins_s >= (1LL << 30) || bins_i >= (1LL << 30) || items_s >= (1LL << 30) || items_i >= (1LL << 30))
 			return set_error(IBK_ERR_INVALID_ARGUMENT, "batch has too many tiles");
-		smem_max = std::max(smem_max, spread_tile_bytes(bi.g, bi.ts, b.M, b.precision));
+		smem_max = std::max(smem_max, spread_tile_bytes(bi.g, bi.ts, b.delta_kind, b.delta_order, b.M, b.precision));
 		dense_max = std::max(dense_max, dense_tile_bytes(bi.ts, b.dims));
 		limit_max = std::max(limit_max, spread_limit_bytes(bi.g, bi.ts, b.M, b.precision));
 		region_max = std::max(region_max, interp_region_bytes(bi.g, bi.ti, b.M));

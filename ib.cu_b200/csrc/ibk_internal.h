@@ -91,7 +91,7 @@ constexpr int kMaxTileExtent = 64;
 // Shared memory of a spread CTA for tiles tg, what of it counts against the
 // limit on tile shapes, and an interpolation CTA's staged region (largest
 // component, stencil width M), in bytes.
-size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision);
+size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int kind, int order, int M, int precision);
 size_t dense_tile_bytes(const TileGeom& tg, int dims);     // of a dense FP32C spread CTA
 size_t spread_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision);
 size_t interp_region_bytes(const GridGeom& g, const TileGeom& tg, int M);
@@ -128,7 +128,7 @@ ibk_status set_error(ibk_status s, const std::string& msg);
 ibk_status check_launch(const char* what);
 
 // The most dynamic shared memory that any launch takes: tile shapes are held
-// to 200 KB, beside which an FP64 spread stages up to 10.5 KB of weights; with
+// to 200 KB, beside which an FP64 spread stages 7.5 KB of weights; with
 // the kernels' static shared memory it stays below the 227 KB of a CTA.
 constexpr int kMaxDynamicSmem = 216 * 1024;
 

@@ -127,31 +127,43 @@ ibk_status bin_points(Plan& plan, const OpArgs& a, const TileGeom& tg, Binned& o
 	return IBK_OK;
 }
 
+// An FP64 spread; parts > 1: as many CTAs share a tile's candidates (owners
+// only) and add their sums to zeroed faces.
+template <typename D, int DIMS, bool OWNERS>
+ibk_status launch_spread64(Plan& plan, const OpArgs& a, const TileGeom& tg, const Binned& b, const double* fl, CompPtrs fe,
+                           int parts = 1)
+{
+	const size_t smem = spread_smem_bytes(*a.g, tg, D::M, IBK_PRECISION_FP64, OWNERS);
+	auto kern = spread_tile64_kernel<D, DIMS, OWNERS>;
+	ibk_status s = allow_smem(kern);
+	if (s != IBK_OK) return s;
+	for (int c = 0; c < DIMS && parts > 1; ++c) {
+		cudaError_t e = cudaMemsetAsync(fe.p[c], 0, sizeof(double) * (size_t) a.g->comp[c].size, a.stream);
+		if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+	}
+	return launch(plan, "spread_tile_kernel", a.stream, [&] {
+		kern<<<dim3(tg.num_tiles, DIMS, parts), s64_threads<OWNERS>(), smem, a.stream>>>(*a.g, tg, a.n, a.x, fl, b.recs,
+		                                                                                b.off, fe);
+	});
+}
+
 template <typename D, int DIMS, int PREC>
 ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const Binned& b, const double* fl, CompPtrs fe)
 {
-	const size_t smem = spread_smem_bytes(*a.g, tg, D::M, PREC);
 	ibk_status s;
 	if constexpr (PREC == IBK_PRECISION_FP64) {
-		auto kern = spread_tile64_kernel<D, DIMS>;
-		if ((s = allow_smem(kern)) != IBK_OK) return s;
-		// Few tiles with many candidates each (about 2.5 per point): several
-		// CTAs share a tile's candidates and add their sums to zeroed faces.
-		const long long items = (long long) tg.num_tiles * DIMS, cand = 5LL * a.n / (2 * tg.num_tiles);
-		int parts = 1;
-		if (DIMS == 3 && items < 2LL * plan.num_sms && cand >= kS64SplitCandidates)
-			parts = (int) std::min((4LL * plan.num_sms + items - 1) / items, cand / (kS64SplitCandidates / 4));
-		for (int c = 0; c < DIMS && parts > 1; ++c) {
-			cudaError_t e = cudaMemsetAsync(fe.p[c], 0, sizeof(double) * (size_t) a.g->comp[c].size, a.stream);
-			if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+		if constexpr (s64_owners<D, DIMS>()) {
+			const long long items = (long long) tg.num_tiles * DIMS, cand = 5LL * a.n / (2 * tg.num_tiles);
+			if (items < 2LL * plan.num_sms && cand >= kS64SplitCandidates)
+				return launch_spread64<D, DIMS, true>(plan, a, tg, b, fl, fe, (int) std::min(
+					(4LL * plan.num_sms + items - 1) / items, cand / (kS64SplitCandidates / 4)));
+			return launch_spread64<D, DIMS, true>(plan, a, tg, b, fl, fe);
 		}
-		return launch(plan, "spread_tile_kernel", a.stream, [&] {
-			kern<<<dim3(tg.num_tiles, DIMS, parts), s64_threads<DIMS>(), smem, a.stream>>>(*a.g, tg, a.n, a.x, fl, b.recs,
-			                                                                              b.off, fe);
-		});
+		return launch_spread64<D, DIMS, false>(plan, a, tg, b, fl, fe);
 	} else {
 		// one CTA per tile for every component, dense tiles deferred to the
 		// folded kernel
+		const size_t smem = spread_smem_bytes(*a.g, tg, D::M, PREC, false);
 		const bool few = tg.num_tiles <= 2 * plan.num_sms;
 		auto kern = few ? spread_tile_kernel<D, DIMS, kFewThreads> : spread_tile_kernel<D, DIMS>;
 		const int nt = few ? kFewThreads : kTileThreads;
@@ -376,9 +388,9 @@ TileGeom make_tiles(const GridGeom& g, int tag, int M, const int* pref_extent)
 	return tg;
 }
 
-size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
+size_t spread_tile_bytes(const GridGeom& g, const TileGeom& tg, int kind, int order, int M, int precision)
 {
-	return spread_smem_bytes(g, tg, M, precision);
+	return spread_smem_bytes(g, tg, M, precision, spread64_owners(kind, order, g.dims));
 }
 
 size_t dense_tile_bytes(const TileGeom& tg, int dims) { return folded_layout(tg, dims).bytes; }

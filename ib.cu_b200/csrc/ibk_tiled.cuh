@@ -13,7 +13,8 @@
 //            point and summed exactly with 32-bit integer shared atomics
 //            (order-independent; see the fixed-point notes below).
 //     FP64:  one CTA per (tile, component), the reference's exact weights,
-//            FP64 sums in shared memory that one warp owns (spread_tile64).
+//            FP64 sums in shared memory: two owning warps (spread_tile64), or shared
+//            atomics (spread_tile64_atomic).
 //
 // interp_tile  -- one CTA per (tile, component) stages the tile plus the
 //   stencil halo of that component in shared memory with one TMA bulk tensor
@@ -782,6 +783,8 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 }
 
 // ------------------------------------------------------- spread, FP64 ---
+// The cubic B-spline in three dimensions; the other deltas take the form below
+// (spread_tile64_atomic).
 // One CTA per (tile, component).  Two warps each own half of the tile's planes
 // and add a candidate's contributions to them one candidate at a time, a lane
 // per node, by plain loads and stores: no other warp touches those faces and
@@ -815,34 +818,109 @@ __host__ __device__ inline SpreadStrides spread64_strides(int T0, int T1, int T2
 
 // Doubles of staged weights per candidate (odd: the preparing threads' stores
 // then spread over the banks).
-template <int M, int DIMS> constexpr int s64_weights() { return (DIMS * M) | 1; }
+constexpr int kS64Weights = 13;
 
-__host__ __device__ inline size_t spread64_smem_bytes(const GridGeom& g, const TileGeom& tg, int M)
+__host__ __device__ inline size_t spread64_smem_bytes(const GridGeom& g, const TileGeom& tg, bool owners)
 {
-	if (g.dims == 2) return (size_t) spread_strides(tg.T[0], tg.T[1], 1, 2).words * 8;
+	if (!owners) return (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words * 8;
 	const size_t words = (size_t) spread64_strides(tg.T[0], tg.T[1], tg.T[2]).words;
 	// two chunks of weights and, per owner, of entries
-	return words * 8 + 2 * kS64Chunk * ((size_t) ((g.dims * M) | 1) * 8 + kS64Owners * sizeof(int2));
+	return words * 8 + 2 * kS64Chunk * ((size_t) kS64Weights * 8 + kS64Owners * sizeof(int2));
+}
+
+// The weights of the axis' nodes in the tile (bit m of mask), 0 elsewhere.
+template <typename D>
+__device__ __forceinline__ void tile_weights64(double delta, unsigned mask, double* w)
+{
+	constexpr int M = D::M, sh = (M - 1) >> 1;
+	if constexpr (std::is_same_v<D, Delta<kBspline, 3>>) {
+		weights64<D>(delta, w);
+	} else {
+#pragma unroll
+		for (int m = 0; m < M; ++m) w[m] = (mask >> m & 1u) ? D::phi64(__dadd_rn(delta, (double) (m - sh))) : 0.0;
+	}
+}
+
+// Adds a tile's candidates to its accumulators, a thread per candidate, by
+// shared atomics.  Every thread of a CTA of NT calls it.
+template <typename D, int DIMS, int NT>
+__device__ __forceinline__ void add_candidates64(const GridGeom& g, const TileGeom& tg, int n, const double* __restrict__ x,
+                                                 const double* __restrict__ fl, const PointRec* __restrict__ recs, int pbase,
+                                                 const RangeTable& rt, int ncand, int c, const int* e, const SpreadStrides& ss,
+                                                 double* acc)
+{
+	constexpr int M = D::M, sh = (M - 1) >> 1;
+	const CompGeom& cg = g.comp[c];
+	int cells[3] = {1, 1, 1};
+	bool wrap[3] = {false, false, false}, wrap_any = false;
+#pragma unroll
+	for (int d = 0; d < DIMS; ++d) {
+		cells[d] = tg.cells[d];
+		wrap[d] = !g.solid[d] && tg.ntiles[d] == 1;
+		wrap_any = wrap_any || wrap[d];
+	}
+	int r = 0;
+	for (int it = threadIdx.x; it < ncand; it += NT) {
+		const PointRec rec = load_rec(recs + range_walk(rt, r, it));
+		const int sft = rt.shift[r], p = rec.p - pbase;
+		int l[DIMS];
+		unsigned mk[DIMS];
+		bool any = true;
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d) {
+			l[d] = rec_origin(rec.org, d) + unpack8(sft, d) + (tg.tag_mac && d == c ? rec_own_shift(rec.org, d) : 0);
+			mk[d] = wrap[d] ? (1u << M) - 1u : axis_mask<M>(l[d] - sh, e[d]);
+			any = any && mk[d] != 0u;
+		}
+		if (!any) continue;
+		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
+		double w[DIMS][M];
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d)
+			tile_weights64<D>(axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta, mk[d], w[d]);
+#pragma unroll
+		for (int m0 = 0; m0 < M; ++m0) w[0][m0] = __dmul_rn(w[0][m0], f);
+		if (!wrap_any) {
+			double* first = acc + (l[0] - sh) + (l[1] - sh) * ss.S1 + (DIMS == 3 ? (l[2] - sh) * ss.S2 : 0);
+			constexpr int R = DIMS == 3 ? M * M : M;
+#pragma unroll
+			for (int q = 0; q < R; ++q) {
+				const int m1 = q % M, m2 = q / M;
+				const unsigned rm = DIMS == 3 ? (mk[1] >> m1) & (mk[2] >> m2) & 1u : (mk[1] >> m1) & 1u;
+				if (!rm) continue;
+				const double w12 = DIMS == 3 ? __dmul_rn(w[1][m1], w[DIMS - 1][m2]) : w[1][m1];
+				double* row = first + m1 * ss.S1 + (DIMS == 3 ? m2 * ss.S2 : 0);
+#pragma unroll
+				for (int m0 = 0; m0 < M; ++m0)
+					if ((mk[0] >> m0) & 1u) atomicAdd(row + m0, __dmul_rn(w[0][m0], w12));
+			}
+		} else {
+			spread_wrapped<D, DIMS>(l, e, cells, wrap, ss.S1, ss.S2, [&](int li, double v) { atomicAdd(acc + li, v); },
+				[&](int m0, int m1, int m2) {
+					return __dmul_rn(w[0][m0], DIMS == 3 ? __dmul_rn(w[1][m1], w[DIMS - 1][m2]) : w[1][m1]);
+				});
+		}
+	}
 }
 
 // part of parts: this CTA's share of the candidates (parts > 1: sums are added
 // to faces that the caller has zeroed).
-template <typename D, int DIMS>
+template <typename D>
 __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom& tg, int n,
                                               const double* __restrict__ x, const double* __restrict__ fl,
                                               const PointRec* __restrict__ recs, int pbase,
                                               const int* __restrict__ off, const CompPtrs& fe, int tile, int c, int part, int parts)
 {
-	constexpr int M = D::M, sh = (M - 1) >> 1, LAST = DIMS - 1;
-	constexpr int W = s64_weights<M, DIMS>();
-	constexpr int NODES = ipow_c(M, DIMS), ROUNDS = (NODES + 31) / 32;
+	constexpr int M = D::M, sh = (M - 1) >> 1, DIMS = 3, LAST = DIMS - 1;
+	static_assert(M == 4, "a lane takes two of 64 nodes");
+	constexpr int W = kS64Weights, ROUNDS = 2;
 	constexpr unsigned kAll = (1u << M) - 1u;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ RangeTable rt;
 
 	__shared__ int counts[2][kS64Owners];        // entries per chunk buffer and owner
 
-	const SpreadStrides ss = spread64_strides(tg.T[0], tg.T[1], DIMS == 3 ? tg.T[2] : 1);
+	const SpreadStrides ss = spread64_strides(tg.T[0], tg.T[1], tg.T[2]);
 	double* acc = reinterpret_cast<double*>(smem_raw);
 	double* weights = acc + ss.words;
 	int2* entries = reinterpret_cast<int2*>(weights + 2 * kS64Chunk * W);    // [buffer][owner][entry], on 16 bytes
@@ -868,7 +946,7 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const bool owner = warp < kS64Owners;
 	const int maker = warp - kS64Owners;
-	const int quarter = (tg.T[LAST] + kS64Owners - 1) / kS64Owners;     // an owner's faces along the last axis
+	const int share = (tg.T[LAST] + kS64Owners - 1) / kS64Owners;       // an owner's faces along the last axis
 
 	// A prepared candidate: its first node (an offset into the tile, or per
 	// axis where a node may wrap), the masks of the nodes that the owners take
@@ -907,9 +985,9 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 				for (int h = 0; h < kS64Owners; ++h) {
 					if (wrap) {
 						for (int m = 0; m < M; ++m)
-							last[h] |= (unsigned) (wrap_index(j0 + m, tg.cells[d]) / quarter == h) << m;
+							last[h] |= (unsigned) (wrap_index(j0 + m, tg.cells[d]) / share == h) << m;
 					} else {
-						last[h] = mk & axis_mask<M>(j0 - h * quarter, quarter);
+						last[h] = mk & axis_mask<M>(j0 - h * share, share);
 					}
 				}
 			}
@@ -945,21 +1023,15 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 		}
 	};
 
-	// this lane's node of each round: its axis indices and its bits of the
-	// entries' masks (a lane without a node has a bit that none holds); a
-	// 4-point stencil's rounds differ in the last index only
-	constexpr bool ALIKE = DIMS == 3 && 32 % (M * M) == 0;
-	int m0[ROUNDS], m1[ROUNDS], m2[ROUNDS];
+	// this lane's nodes, which differ in the last index only: their axis indices
+	// and their bits of the entries' masks
+	const int m0 = lane % M, m1 = lane / M % M;
+	int m2[ROUNDS];
 	unsigned bits[ROUNDS];
 #pragma unroll
 	for (int q = 0; q < ROUNDS; ++q) {
-		const int v = (ALIKE ? 0 : q * 32) + lane;
-		m0[q] = v % M;
-		m1[q] = (v / M) % M;
-		m2[q] = DIMS == 3 ? v / (M * M) + (ALIKE ? q * (32 / (M * M)) : 0) : 0;
-		const bool none = !ALIKE && v >= NODES;
-		bits[q] = none ? 1u << 31 : 1u << m0[q] | 1u << (8 + m1[q]) | (DIMS == 3 ? 1u << (16 + m2[q]) : 0u);
-		if (none) m0[q] = m1[q] = m2[q] = 0;
+		m2[q] = lane / (M * M) + q * (32 / (M * M));
+		bits[q] = 1u << m0 | 1u << (8 + m1) | 1u << (16 + m2[q]);
 	}
 	auto add = [&](auto wrapped, int chunk) {
 		constexpr bool WRAP = decltype(wrapped)::value;
@@ -970,19 +1042,17 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 		// The candidates go two by two: of a pair's work only the load - add -
 		// store of one after the other's is a chain, the rest is for the next
 		// pair and hides behind it.  An odd list ends with an empty entry.
-		double wa[2][ROUNDS], wy[2][ROUNDS], wz[2][ROUNDS];
+		double wa[2], wy[2], wz[2][ROUNDS];
 		int at[2][ROUNDS];
 		bool on[2][ROUNDS];
 		auto fetch = [&](int4 two) {            // a pair's weights
 #pragma unroll
 			for (int u = 0; u < 2; ++u) {
 				const double* q = wb + ((unsigned) (u ? two.w : two.y) >> 24) * W;
+				wa[u] = q[m0];
+				wy[u] = q[M + m1];
 #pragma unroll
-				for (int i = 0; i < ROUNDS; ++i) {
-					wa[u][i] = ALIKE && i ? wa[u][0] : q[m0[i]];
-					wy[u][i] = ALIKE && i ? wy[u][0] : q[M + m1[i]];
-					wz[u][i] = DIMS == 3 ? q[2 * M + m2[i]] : 1.0;
-				}
+				for (int i = 0; i < ROUNDS; ++i) wz[u][i] = q[2 * M + m2[i]];
 			}
 		};
 		auto locate = [&](int4 two) {           // its nodes
@@ -994,14 +1064,14 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 				for (int i = 0; i < ROUNDS; ++i) {
 					on[u][i] = (~mask & bits[i]) == 0u;
 					if constexpr (WRAP) {
-						const int a0 = (first & 255) - 128 + m0[i], a1 = ((first >> 8) & 255) - 128 + m1[i];
-						const int a2 = DIMS == 3 ? ((first >> 16) & 255) - 128 + m2[i] : 0;
+						const int a0 = (first & 255) - 128 + m0, a1 = ((first >> 8) & 255) - 128 + m1;
+						const int a2 = ((first >> 16) & 255) - 128 + m2[i];
 						const bool w0 = !g.solid[0] && tg.ntiles[0] == 1, w1 = !g.solid[1] && tg.ntiles[1] == 1;
-						const bool w2 = DIMS == 3 && !g.solid[2] && tg.ntiles[2] == 1;
+						const bool w2 = !g.solid[2] && tg.ntiles[2] == 1;
 						at[u][i] = (w0 ? wrap_index(a0, tg.cells[0]) : a0) + (w1 ? wrap_index(a1, tg.cells[1]) : a1) * ss.S1 +
 						           (w2 ? wrap_index(a2, tg.cells[2]) : a2) * ss.S2;
 					} else {
-						at[u][i] = first + m0[i] + m1[i] * ss.S1 + m2[i] * ss.S2;
+						at[u][i] = first + m0 + m1 * ss.S1 + m2[i] * ss.S2;
 					}
 				}
 			}
@@ -1021,7 +1091,7 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 			for (int u = 0; u < 2; ++u)
 #pragma unroll
 				for (int i = 0; i < ROUNDS; ++i)
-					t[u][i] = __dmul_rn(wa[u][i], DIMS == 3 ? __dmul_rn(wy[u][i], wz[u][i]) : wy[u][i]);
+					t[u][i] = __dmul_rn(wa[u], __dmul_rn(wy[u], wz[u][i]));
 			next = pairs[min(j + 1, npairs - 1)];
 #pragma unroll
 			for (int i = 0; i < ROUNDS; ++i)
@@ -1069,86 +1139,69 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 	}
 }
 
-// Two dimensions: one CTA of kTileThreads per (tile, component), a thread per
-// candidate, FP64 shared atomics.  A stencil has at most 36 nodes and a tile
-// few faces, so the owners of spread_tile64 would work through a long chain
-// with half of their lanes idle (24 outlines of 160 points on 240 x 120 cells:
-// 20 us against 30).
-template <typename D>
-__device__ __forceinline__ void spread_tile64_plane(const GridGeom& g, const TileGeom& tg, int n,
-                                                    const double* __restrict__ x, const double* __restrict__ fl,
-                                                    const PointRec* __restrict__ recs, int pbase,
-                                                    const int* __restrict__ off, const CompPtrs& fe, int tile, int c)
+// The other form: one CTA of kTileThreads per (tile, component), a thread per
+// candidate, FP64 shared atomics.  Every delta but the cubic B-spline takes
+// it: the owners' lanes are 64 nodes in two rounds, and two warps cannot
+// prepare dearer weights in time.  128 x 64 x 128 cells, 124,700 points, in us,
+// binning included, a general form of the owners / this one: bspline<1> 104 /
+// 59, bspline<2> 134 / 99, bspline<4> 1589 / 541, bspline<5> 7162 / 2107, peskin
+// 223 / 180, roma 214 / 111, cosine 272 / 195, hat 102 / 58.  In two dimensions
+// a stencil has at most 36 nodes and a tile few faces, so the owners would
+// work through a long chain with half of their lanes idle (24 outlines of 160
+// points on 240 x 120 cells: 20 us against 30).
+template <typename D, int DIMS>
+__device__ __forceinline__ void spread_tile64_atomic(const GridGeom& g, const TileGeom& tg, int n,
+                                                     const double* __restrict__ x, const double* __restrict__ fl,
+                                                     const PointRec* __restrict__ recs, int pbase,
+                                                     const int* __restrict__ off, const CompPtrs& fe, int tile, int c)
 {
-	constexpr int M = D::M, sh = (M - 1) >> 1;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ RangeTable rt;
-	const SpreadStrides ss = spread_strides(tg.T[0], tg.T[1], 1, 2);
+	const SpreadStrides ss = spread_strides(tg.T[0], tg.T[1], DIMS == 3 ? tg.T[2] : 1, DIMS);
 	double* acc = reinterpret_cast<double*>(smem_raw);
 	const CompGeom& cg = g.comp[c];
 	int tc[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, e[3] = {1, 1, 1};
-	bool wrap[2];
 	tile_coords(tg, tile, tc);
 #pragma unroll
-	for (int d = 0; d < 2; ++d) {
+	for (int d = 0; d < DIMS; ++d) {
 		lo[d] = tc[d] * tg.T[d];
 		e[d] = min(tg.T[d], cg.points[d] - lo[d]);
-		wrap[d] = !g.solid[d] && tg.ntiles[d] == 1;
 	}
-	build_ranges<2>(g, tg, tc, off, rt);
+	build_ranges<DIMS>(g, tg, tc, off, rt);
 	const int ncand = rt.pref[rt.count];
-	for (int i = threadIdx.x; i < ss.words; i += kTileThreads) acc[i] = 0.0;
-	__syncthreads();
-	int r = 0;
-	for (int it = threadIdx.x; it < ncand; it += kTileThreads) {
-		const PointRec rec = load_rec(recs + range_walk(rt, r, it));
-		const int sft = rt.shift[r], p = rec.p - pbase;
-		double w[2][M];
-		int at[2][M];
-		unsigned mk[2] = {0u, 0u};
-#pragma unroll
-		for (int d = 0; d < 2; ++d) {
-			const int j0 = rec_origin(rec.org, d) + unpack8(sft, d) + (tg.tag_mac && d == c ? rec_own_shift(rec.org, d) : 0) - sh;
-#pragma unroll
-			for (int m = 0; m < M; ++m) {
-				bool in;
-				at[d][m] = local_node(j0 + m, e[d], tg.cells[d], wrap[d], in);
-				mk[d] |= (unsigned) in << m;
-			}
-		}
-		if (mk[0] == 0u || mk[1] == 0u) continue;
-#pragma unroll
-		for (int d = 0; d < 2; ++d) weights64<D>(axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta, w[d]);
-		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
-#pragma unroll
-		for (int m1 = 0; m1 < M; ++m1)
-#pragma unroll
-			for (int m0 = 0; m0 < M; ++m0)
-				if ((mk[0] >> m0) & (mk[1] >> m1) & 1u)
-					atomicAdd(acc + at[1][m1] * ss.S1 + at[0][m0], __dmul_rn(__dmul_rn(w[0][m0], f), w[1][m1]));
+	if (ncand == 0) {
+		write_tile<DIMS, kTileThreads>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [](int) { return 0.0; });
+		return;
 	}
+	for (int i = threadIdx.x * 2; i < ss.words; i += kTileThreads * 2)      // words: a multiple of 4
+		*reinterpret_cast<double2*>(acc + i) = make_double2(0.0, 0.0);
 	__syncthreads();
-	write_tile<2, kTileThreads>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [&](int li) { return acc[li]; });
+	add_candidates64<D, DIMS, kTileThreads>(g, tg, n, x, fl, recs, pbase, rt, ncand, c, e, ss, acc);
+	__syncthreads();
+	write_tile<DIMS, kTileThreads>(fe.p[c], cg, lo, e, ss.S1, ss.S2, [&](int li) { return acc[li]; });
 }
 
-// Threads and one tile of the FP64 spread kernels.
-template <int DIMS> constexpr int s64_threads() { return DIMS == 3 ? kS64Threads : kTileThreads; }
+// The form for a delta and its CTAs: threads and CTAs per SM.
+constexpr bool spread64_owners(int kind, int order, int dims) { return kind == kBspline && order == 3 && dims == 3; }
+template <typename D, int DIMS> constexpr bool s64_owners() { return DIMS == 3 && std::is_same_v<D, Delta<kBspline, 3>>; }
+template <bool OWNERS> constexpr int s64_threads() { return OWNERS ? kS64Threads : kTileThreads; }
+template <bool OWNERS> constexpr int s64_ctas() { return OWNERS ? 4 : 3; }
 
-template <typename D, int DIMS>
+template <typename D, int DIMS, bool OWNERS>
 __device__ __forceinline__ void spread_any64(const GridGeom& g, const TileGeom& tg, int n, const double* __restrict__ x,
                                              const double* __restrict__ fl, const PointRec* __restrict__ recs, int pbase,
                                              const int* __restrict__ off, const CompPtrs& fe, int tile, int c, int part = 0,
                                              int parts = 1)
 {
-	if constexpr (DIMS == 3) spread_tile64<D, 3>(g, tg, n, x, fl, recs, pbase, off, fe, tile, c, part, parts);
-	else spread_tile64_plane<D>(g, tg, n, x, fl, recs, pbase, off, fe, tile, c);
+	if constexpr (OWNERS) spread_tile64<D>(g, tg, n, x, fl, recs, pbase, off, fe, tile, c, part, parts);
+	else spread_tile64_atomic<D, DIMS>(g, tg, n, x, fl, recs, pbase, off, fe, tile, c);
 }
 
 // Shared memory of a spread CTA.  FP32C: every component's accumulator words
 // (4 bytes per face; the occupancy grid where larger) between guard words.
-__host__ __device__ inline size_t spread_smem_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
+__host__ __device__ inline size_t spread_smem_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision, bool owners)
 {
-	if (precision != IBK_PRECISION_FP32C) return spread64_smem_bytes(g, tg, M);
+	if (precision != IBK_PRECISION_FP32C) return spread64_smem_bytes(g, tg, owners);
 	const size_t words = (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words;
 	const size_t occ = occupancy_words_rt(g, tg, M), acc = words * 3;
 	return ((acc > occ ? acc : occ) + 2 * kGuardWords) * 4;
@@ -1158,7 +1211,7 @@ __host__ __device__ inline size_t spread_smem_bytes(const GridGeom& g, const Til
 // component in FP64).
 __host__ __device__ inline size_t spread_tile_limit_bytes(const GridGeom& g, const TileGeom& tg, int M, int precision)
 {
-	if (precision == IBK_PRECISION_FP32C) return spread_smem_bytes(g, tg, M, precision) - 4 * kGuardWords;
+	if (precision == IBK_PRECISION_FP32C) return spread_smem_bytes(g, tg, M, precision, false) - 4 * kGuardWords;
 	return (size_t) spread_strides(tg.T[0], tg.T[1], tg.T[2], g.dims).words * 8 + 4 * kGuardWords;
 }
 
@@ -1173,13 +1226,14 @@ spread_tile_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, c
 	spread_tile<D, DIMS, false, NT>(g, tg, recs, forces, off, fe, blockIdx.x, -1, defer, blockIdx.x);
 }
 
-// grid: (tile, component, part); four CTAs of 52 KB per SM at 16^3 tiles.
-template <typename D, int DIMS>
-__global__ void __launch_bounds__(s64_threads<DIMS>(), 4)
+// grid: (tile, component, part); of the owners' form four CTAs of 52 KB per SM
+// at 16^3 tiles, of the other three (85 registers).
+template <typename D, int DIMS, bool OWNERS>
+__global__ void __launch_bounds__(s64_threads<OWNERS>(), s64_ctas<OWNERS>())
 spread_tile64_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x, const double* __restrict__ fl,
                      const PointRec* __restrict__ recs, const int* __restrict__ off, CompPtrs fe)
 {
-	spread_any64<D, DIMS>(g, tg, n, x, fl, recs, 0, off, fe, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
+	spread_any64<D, DIMS, OWNERS>(g, tg, n, x, fl, recs, 0, off, fe, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
 }
 
 // The deferred dense tiles of an FP32C spread, folded (see Deferral); the
