@@ -19,9 +19,19 @@ constexpr int kThreads = 128;
 // difference, and with 1024 threads 94 and 62).
 constexpr int kFewThreads = 512;
 
-// Candidates of an average tile from which the FP64 spread splits them (30^3
-// cells, 416,000 points: 0.71 ms against 1.66 ms with shared atomics).
-constexpr int kS64SplitCandidates = 4096;
+// The FP64 spread of the cubic B-spline, by the candidates of an average tile
+// (about 2.5 per point), in us, binning included, n points on cells^3:
+//   owners, the candidates split over several CTAs, where the tiles are few
+//   and full (132,600 points on 26^3: 257, unsplit atomics 678; on 32^3: 248, 379);
+//   atomics where the tiles are fewer than the SMs and have many candidates all
+//   the same, since then the time is that of the longest chain (22,100 on 26^3:
+//   160, owners 199; 132,600 on 40^3: 266, 297, and on 72^3: 243, 286), and where
+//   tiles of more than kS64SmallTile cells have few, often in clumps (11,050
+//   points on 96^3: 84, 99; 2,210 on 160^3: 82, 93; but 8,832 of one finely
+//   sampled cell on 96^3: 187, 166);
+//   owners else (1.36 M points on 256 x 128 x 256: 1009, atomics 1036; 124,700
+//   on 128 x 64 x 128: 166, 173; 8,832 on 64^3 in small tiles: 91, 101).
+constexpr int kS64SplitCandidates = 4096, kS64ManyCandidates = 800, kS64FewCandidates = 160, kS64SmallTile = 2048;
 
 inline int blocks_for(long long n, int threads) { return (int) ((n + threads - 1) / threads); }
 
@@ -157,7 +167,9 @@ ibk_status launch_spread(Plan& plan, const OpArgs& a, const TileGeom& tg, const 
 			if (items < 2LL * plan.num_sms && cand >= kS64SplitCandidates)
 				return launch_spread64<D, DIMS, true>(plan, a, tg, b, fl, fe, (int) std::min(
 					(4LL * plan.num_sms + items - 1) / items, cand / (kS64SplitCandidates / 4)));
-			return launch_spread64<D, DIMS, true>(plan, a, tg, b, fl, fe);
+			const bool few = tg.num_tiles < plan.num_sms, small = tg.T[0] * tg.T[1] * tg.T[2] <= kS64SmallTile;
+			if (few ? cand < kS64ManyCandidates : small || cand >= kS64FewCandidates)
+				return launch_spread64<D, DIMS, true>(plan, a, tg, b, fl, fe);
 		}
 		return launch_spread64<D, DIMS, false>(plan, a, tg, b, fl, fe);
 	} else {

@@ -784,7 +784,7 @@ __device__ __forceinline__ void spread_tile(const GridGeom& g, const TileGeom& t
 
 // ------------------------------------------------------- spread, FP64 ---
 // The cubic B-spline in three dimensions; the other deltas take the form below
-// (spread_tile64_atomic).
+// (spread_tile64_atomic), and so does this one where the host's rule says so.
 // One CTA per (tile, component).  Two warps each own half of the tile's planes
 // and add a candidate's contributions to them one candidate at a time, a lane
 // per node, by plain loads and stores: no other warp touches those faces and
@@ -1140,8 +1140,8 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 }
 
 // The other form: one CTA of kTileThreads per (tile, component), a thread per
-// candidate, FP64 shared atomics.  Every delta but the cubic B-spline takes
-// it: the owners' lanes are 64 nodes in two rounds, and two warps cannot
+// candidate, FP64 shared atomics.  Every delta but the cubic B-spline always
+// takes it: the owners' lanes are 64 nodes in two rounds, and two warps cannot
 // prepare dearer weights in time.  128 x 64 x 128 cells, 124,700 points, in us,
 // binning included, a general form of the owners / this one: bspline<1> 104 /
 // 59, bspline<2> 134 / 99, bspline<4> 1589 / 541, bspline<5> 7162 / 2107, peskin

@@ -96,3 +96,18 @@ def test_positions_beyond_the_index_range(ibk, oracle, cuda, tiles):
     assert np.array_equal(ul[:, n:], np.zeros((3, far)))
     want, ua = oracle.interpolate(g, np.concatenate(near), ue, with_abs=True)
     check_interp(np.ascontiguousarray(ul[:, :n]).reshape(-1), want, ua)
+
+
+# both forms of the cubic B-spline's spread on either side of the rules between
+# them, at tiles that split unevenly, are not padded or wrap: (cells, tiles, points)
+@pytest.mark.parametrize("cells,tiles,n", [
+    ((24, 24, 24), None, 60000),                    # few full tiles: split candidates
+    ((24, 24, 24), None, 8000), ((24, 24, 24), None, 9000),                 # 27 tiles, below and above the limit of few
+    ((128, 128, 128), None, 30000), ((128, 128, 128), None, 34000),         # 512 of 16^3, likewise
+    ((128, 128, 128), (20, 20, 20), 24000), ((128, 128, 128), (32, 24, 18), 24000),
+    ((128, 128, 128), (13, 11, 13), 3000), ((16, 128, 128), (16, 8, 8), 3000), ((16, 16, 16), (16, 16, 16), 9000)])
+def test_cubic_forms(ibk, oracle, cuda, cells, tiles, n):
+    rng = np.random.default_rng(n)
+    L = [c / 40.0 for c in cells]
+    x = np.concatenate([rng.uniform(-0.01, l + 0.01, n) for l in L])
+    _run(ibk, oracle, cuda, x, L, [0, 1, 0], min(cells), tiles=tiles)
