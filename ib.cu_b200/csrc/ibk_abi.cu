@@ -281,9 +281,15 @@ ibk_status ibk_plan_create(const ibk_domain* domain, int tag, int refinement, ib
 	// four per axis): a tile's candidates are a serial chain there (one red cell
 	// on 64^3, 64 tiles of 16^3, both operators: 95 -> 81 us).  Not where x would
 	// get an odd extent, whose regions the interpolation cannot stage by TMA
-	// (110 x 110 x 220 cells in tiles of 13: 143 instead of 105 us).
+	// (110 x 110 x 220 cells in tiles of 13: 143 instead of 105 us).  Nor for
+	// stencils of two points, whose spread is too short to pay for more tiles (2,210
+	// points on 64^3: 33 -> 36 us), and of five and six, which reach too many
+	// small ones (132,600 points on 80^3, bspline<4>: spread 795 -> 870,
+	// interpolation 212 -> 227 us; 22,100 on 64^3, bspline<5>: 768 -> 878, 224 ->
+	// 252 us).
 	plan->tiles = make_tiles(g, tag, info.meshwidths);
-	if (precision == IBK_PRECISION_FP64 && dims == 3 && plan->tiles.num_tiles <= plan->num_sms) {
+	const int M = info.meshwidths;
+	if (precision == IBK_PRECISION_FP64 && dims == 3 && (M == 3 || M == 4) && plan->tiles.num_tiles <= plan->num_sms) {
 		int small[kMaxDims];
 		for (int d = 0; d < dims; ++d) small[d] = std::min(16, std::max(8, g.comp[0].cells[d] / 8));
 		const TileGeom t = make_tiles(g, tag, info.meshwidths, small);
