@@ -408,7 +408,9 @@ direction_kernel(long long n, const double* __restrict__ sc, const double* __res
 // iteration: 48 + 32 bytes (one kernel per operator product, update and
 // direction moved 152).  The products use fused multiply-adds with lambda
 // folded into the coefficients; the operators themselves
-// (march_apply_kernel) keep the reference's operation order.
+// (march_apply_kernel) keep the reference's operation order.  Grids of two
+// dimensions have kernels of their own (direction_plane_kernel,
+// polynomial_plane_kernel): one plane, nothing to march.
 
 // Index of an extended coordinate on an axis: wrapped on a periodic axis, -1
 // outside a wall.
@@ -516,6 +518,10 @@ struct UniformH {
 		return __fma_rn(centre, c, side * (((xm + xp) + (ym + yp)) + zm));
 	}
 	__device__ __forceinline__ double top(int, int) const { return side; }
+	__device__ __forceinline__ double plane(int, double c, double xm, double xp, double ym, double yp) const
+	{
+		return __fma_rn(centre, c, side * ((xm + xp) + (ym + yp)));
+	}
 };
 
 // walls along y only (a channel),
@@ -554,11 +560,52 @@ struct GeneralH {
 	__device__ __forceinline__ double top(int row, int plane) const { return x.id * yt[row].id * zt[plane].hi; }
 };
 
+// In two dimensions H at a face is one expression, plane(): UniformH's, or this
+// one where the block reaches a wall.
+struct PlaneH {
+	AxisCoef x;
+	const AxisCoef* yt;
+	__device__ __forceinline__ PlaneH(const AxisCoef& cx, const AxisCoef* y) : x(cx), yt(y) {}
+	__device__ __forceinline__ double plane(int row, double c, double xm, double xp, double ym, double yp) const
+	{
+		const AxisCoef y = yt[row];
+		const double ax = __fma_rn(x.hi, xp, __fma_rn(x.lo, xm, (x.id + x.diag) * c));
+		const double ay = __fma_rn(y.hi, yp, __fma_rn(y.lo, ym, y.diag * c));
+		return __fma_rn(x.id, ay, y.id * ax);
+	}
+};
+
 // The coefficients of `count` faces from `first` on along an axis.
 __device__ __forceinline__ void fill_table(const FluidOps& o, int axis, int first, int count, AxisCoef* t)
 {
 	for (int i = threadIdx.x; i < count; i += blockDim.x)
 		t[i] = axis_coef(o.ax[axis], axis < o.dims, o.lambda, fold_index(o.ax[axis], first + i));
+}
+
+// After a direction: the loop test of pcg.h:21, then alpha or the bail-out of
+// pcg.h:23-31; sums: d . H d and d . d.
+__device__ __forceinline__ void judge(const double* sums, double* sc, double tol, int max_iterations, double* host)
+{
+	sc[1] = sums[0];
+	sc[2] = sums[1];
+	if (!(sqrt(sums[1]) > tol)) sc[5] = kConverged;
+	else if (sc[6] >= (double) max_iterations) sc[5] = kLimit;
+	else if (fabs(sums[0]) < tol * tol) sc[5] = kBailOut;
+	else sc[3] = sc[0] / sums[0];
+	host[0] = sc[5];
+	host[1] = sc[6];
+}
+
+// After a polynomial: delta = r . z, and beta but for the first.
+__device__ __forceinline__ void advance(double delta, double* sc, int first)
+{
+	if (first) {
+		sc[0] = delta;              // pcg.h:14-18: delta = r . d
+	} else {
+		sc[4] = delta / sc[0];      // pcg.h:36-39: beta = delta' / delta
+		sc[0] = delta;
+		sc[6] += 1.0;
+	}
 }
 
 // Time of one step of polynomial_kernel's wide tile over the small tile's, from
@@ -693,16 +740,76 @@ direction_apply_kernel(FluidOps o, double* __restrict__ sc, const double* __rest
 		else
 			march(GeneralH(o, cx, yt, zt));     // the first barrier comes before the tables are read
 	}
-	if (!grid_sums<kDirThreads, 2>(sums, part, done) || threadIdx.x != 0) return;
-	// the loop test of pcg.h:21, then alpha or the bail-out of pcg.h:23-31
-	sc[1] = sums[0];
-	sc[2] = sums[1];
-	if (!(sqrt(sums[1]) > tol)) sc[5] = kConverged;
-	else if (sc[6] >= (double) max_iterations) sc[5] = kLimit;
-	else if (fabs(sums[0]) < tol * tol) sc[5] = kBailOut;
-	else sc[3] = sc[0] / sums[0];
-	host[0] = sc[5];
-	host[1] = sc[6];
+	if (grid_sums<kDirThreads, 2>(sums, part, done) && threadIdx.x == 0) judge(sums, sc, tol, max_iterations, host);
+}
+
+// The same in two dimensions: one plane, no march, the arrays mostly in L2.
+__global__ void __launch_bounds__(kDirThreads, 4)
+direction_plane_kernel(FluidOps o, double* __restrict__ sc, const double* __restrict__ z,
+                       const double* __restrict__ dold, double* __restrict__ dnew, double* __restrict__ x,
+                       double* __restrict__ q, double* __restrict__ part, unsigned* __restrict__ done, int first,
+                       double tol, int max_iterations, double* __restrict__ host)
+{
+	if (sc[5] != 0.0) return;
+	__shared__ double plane[(kDirY + 2) * kDirStride];
+	__shared__ AxisCoef yt[kDirY];
+	const double alpha = sc[3], beta = sc[4];
+	const int P0 = o.ax[0].P, P1 = o.ax[1].P;
+	const int tx = threadIdx.x % kDirX, ty = threadIdx.x / kDirX;
+	const int x0 = blockIdx.x * kDirX, y0 = blockIdx.y * kDirY;
+	const int gi = fold_index(o.ax[0], x0 + tx);
+	const int slot = (ty * kDirRows + 1) * kDirStride + tx + 1;
+	int off[kDirRows];
+	bool own[kDirRows];
+	double v[kDirRows], sums[2] = {0.0, 0.0};
+#pragma unroll
+	for (int c = 0; c < kDirRows; ++c) {
+		const int y = y0 + ty * kDirRows + c, gj = fold_index(o.ax[1], y);
+		const bool on = gi >= 0 && gj >= 0;
+		own[c] = x0 + tx < P0 && y < P1;
+		off[c] = on ? gi + gj * P0 : 0;
+		const double d = on && !first ? __ldg(dold + off[c]) : 0.0;
+		v[c] = __fma_rn(beta, d, on ? __ldg(z + off[c]) : 0.0);
+		plane[slot + c * kDirStride] = v[c];
+		if (own[c]) {
+			dnew[off[c]] = v[c];
+			x[off[c]] = __fma_rn(alpha, d, first ? 0.0 : x[off[c]]);
+		}
+	}
+	if (threadIdx.x < 2 * kDirX + 2 * kDirY) {      // the rows above and below, the columns left and right
+		const int t = threadIdx.x, h = t - 2 * kDirX;
+		const int ex = h < 0 ? t % kDirX : (h < kDirY ? -1 : kDirX);
+		const int ey = h < 0 ? (t < kDirX ? -1 : kDirY) : h % kDirY;
+		const int hi = fold_index(o.ax[0], x0 + ex), hj = fold_index(o.ax[1], y0 + ey);
+		const bool on = hi >= 0 && hj >= 0;
+		const int at = on ? hi + hj * P0 : 0;
+		const double d = on && !first ? __ldg(dold + at) : 0.0;
+		plane[(ey + 1) * kDirStride + ex + 1] = __fma_rn(beta, d, on ? __ldg(z + at) : 0.0);
+	}
+	auto apply = [&](const auto& H) {
+#pragma unroll
+		for (int c = 0; c < kDirRows; ++c) {
+			const int at = slot + c * kDirStride;
+			const double h = H.plane(ty * kDirRows + c, v[c], plane[at - 1], plane[at + 1],
+			                         c > 0 ? v[c - 1] : plane[at - kDirStride],
+			                         c + 1 < kDirRows ? v[c + 1] : plane[at + kDirStride]);
+			if (own[c]) {
+				q[off[c]] = h;
+				sums[0] = __fma_rn(v[c], h, sums[0]);
+				sums[1] = __fma_rn(v[c], v[c], sums[1]);
+			}
+		}
+	};
+	const AxisCoef cx = axis_coef(o.ax[0], true, o.lambda, gi);
+	if (alike(o.ax[0], x0 - 1, x0 + kDirX) && alike(o.ax[1], y0 - 1, y0 + kDirY)) {
+		__syncthreads();
+		apply(UniformH(o, cx, yt, yt));
+	} else {
+		fill_table(o, 1, y0, kDirY, yt);
+		__syncthreads();
+		apply(PlaneH(cx, yt));
+	}
+	if (grid_sums<kDirThreads, 2>(sums, part, done) && threadIdx.x == 0) judge(sums, sc, tol, max_iterations, host);
 }
 
 // polynomial_kernel's tile: EX x TY * ROWS columns, of which the inner ones (a
@@ -721,7 +828,7 @@ template <int EX_, int TY_, int ROWS_, int BLOCKS_>
 struct PolyTile {
 	static constexpr int EX = EX_, TY = TY_, ROWS = ROWS_, BLOCKS = BLOCKS_, HALO = 3;
 	static constexpr int EY = TY * ROWS, X = EX - 2 * HALO, Y = EY - 2 * HALO, THREADS = EX * TY;
-	static constexpr int PLANE = EX * EY, BYTES = 6 * PLANE * (int) sizeof(double);
+	static constexpr int PLANE = EX * EY;
 	static_assert(THREADS % 32 == 0, "whole warps");
 };
 // Of the wide tile's columns 74 % are the block's own, of the small tile's
@@ -731,6 +838,7 @@ struct PolyTile {
 // 117 1.85 against 1.76, 64^3 0.49 against 0.46.
 using PolyWide = PolyTile<64, 8, 4, 1>;
 using PolySmall = PolyTile<32, 16, 1, 2>;
+template <typename T> constexpr int poly_bytes() { return 6 * T::PLANE * (int) sizeof(double); }
 
 struct ChebWeights { double w[4]; };
 
@@ -856,14 +964,89 @@ polynomial_kernel(FluidOps o, double* __restrict__ sc, const double* __restrict_
 		else
 			march(GeneralH(o, cx, yt, zt));
 	}
-	if (!grid_sums<T::THREADS, 1>(sums, part, done) || threadIdx.x != 0) return;
-	if (first) {
-		sc[0] = sums[0];            // pcg.h:14-18: delta = r . d
-	} else {
-		sc[4] = sums[0] / sc[0];    // pcg.h:36-39: beta = delta' / delta
-		sc[0] = sums[0];
-		sc[6] += 1.0;
+	if (grid_sums<T::THREADS, 1>(sums, part, done) && threadIdx.x == 0) advance(sums[0], sc, first);
+}
+
+// The same in two dimensions: the three steps one after the other on the block's
+// columns, a barrier each.  A march of one plane through the kernel above
+// takes seven plane steps, every block of them in GeneralH: a solve of 11
+// iterations on 2400 x 600 faces took 2079 us (one kernel per product, before
+// the fused loop: 1172), now 694; 1000 x 1000 1548 (998), now 534; 240 x 120 304
+// (618), now 252.  Wide against small tiles: 96 x 96 faces 236 / 213 us, 256 x 256
+// 265 / 256 (260 small blocks), 400 x 400 279 / 290 (640), 600 x 600 307 / 380,
+// 2400 x 600 694 / 888.
+using PlaneWide = PolyTile<64, 8, 4, 2>;
+using PlaneSmall = PolyTile<32, 16, 1, 4>;
+
+template <typename T>
+__global__ void __launch_bounds__(T::THREADS, T::BLOCKS)
+polynomial_plane_kernel(FluidOps o, double* __restrict__ sc, const double* __restrict__ r, const double* __restrict__ q,
+                        double* __restrict__ rnew, double* __restrict__ z, double* __restrict__ part,
+                        unsigned* __restrict__ done, int first, ChebWeights cw)
+{
+	if (sc[5] != 0.0) return;
+	__shared__ double planes[2][T::PLANE];      // r' and the second step, the first step
+	__shared__ AxisCoef yt[T::EY];
+	const double alpha = sc[3];
+	const int P0 = o.ax[0].P, P1 = o.ax[1].P;
+	const int tx = threadIdx.x % T::EX, ty = threadIdx.x / T::EX;
+	const int ex0 = (int) blockIdx.x * T::X - T::HALO, ey0 = (int) blockIdx.y * T::Y - T::HALO;
+	const int gi = fold_index(o.ax[0], ex0 + tx);
+	const int slot = ty * T::ROWS * T::EX + tx;
+	const int left = tx > 0 ? -1 : 0, right = tx + 1 < T::EX ? 1 : 0;
+	const int above = ty > 0 ? -T::EX : 0, below = ty + 1 < T::TY ? T::EX : 0;
+	int off[T::ROWS];
+	double v[T::ROWS], sums[1] = {0.0};
+#pragma unroll
+	for (int c = 0; c < T::ROWS; ++c) {
+		const int gj = fold_index(o.ax[1], ey0 + ty * T::ROWS + c);
+		const bool on = gi >= 0 && gj >= 0;
+		off[c] = on ? gi + gj * P0 : 0;
+		v[c] = __fma_rn(-alpha, on && !first ? __ldg(q + off[c]) : 0.0, on ? __ldg(r + off[c]) : 0.0);
+		planes[0][slot + c * T::EX] = v[c];
 	}
+	auto run = [&](const auto& H) {
+		// out = w r' - ws H s, s this thread's columns and their shared copy buf
+		auto step = [&](const double* buf, double w, double ws, const double* s, double* out) {
+#pragma unroll
+			for (int c = 0; c < T::ROWS; ++c) {
+				const int at = slot + c * T::EX;
+				const double h = H.plane(ty * T::ROWS + c, s[c], buf[at + left], buf[at + right],
+				                         c > 0 ? s[c - 1] : buf[at + above],
+				                         c + 1 < T::ROWS ? s[c + 1] : buf[at + below]);
+				out[c] = __fma_rn(w, v[c], -ws * h);
+			}
+		};
+		double a[T::ROWS], b[T::ROWS];
+		__syncthreads();
+		step(planes[0], cw.w[1], cw.w[0], v, a);
+#pragma unroll
+		for (int c = 0; c < T::ROWS; ++c) planes[1][slot + c * T::EX] = a[c];
+		__syncthreads();        // the first step is complete, every read of r' done
+		step(planes[1], cw.w[2], 1.0, a, b);
+#pragma unroll
+		for (int c = 0; c < T::ROWS; ++c) planes[0][slot + c * T::EX] = b[c];
+		__syncthreads();
+		step(planes[0], cw.w[3], 1.0, b, a);
+#pragma unroll
+		for (int c = 0; c < T::ROWS; ++c) {
+			const int ey = ty * T::ROWS + c;
+			if (tx >= T::HALO && tx < T::HALO + T::X && ex0 + tx < P0 && ey >= T::HALO && ey < T::HALO + T::Y &&
+			    ey0 + ey < P1) {
+				rnew[off[c]] = v[c];
+				z[off[c]] = a[c];
+				sums[0] = __fma_rn(v[c], a[c], sums[0]);
+			}
+		}
+	};
+	const AxisCoef cx = axis_coef(o.ax[0], true, o.lambda, gi);
+	if (alike(o.ax[0], ex0, ex0 + T::EX - 1) && alike(o.ax[1], ey0, ey0 + T::EY - 1)) {
+		run(UniformH(o, cx, yt, yt));
+	} else {
+		fill_table(o, 1, ey0, T::EY, yt);       // read after the first barrier
+		run(PlaneH(cx, yt));
+	}
+	if (grid_sums<T::THREADS, 1>(sums, part, done) && threadIdx.x == 0) advance(sums[0], sc, first);
 }
 
 // Planes per block of a tile kernel and the cost that comes with them: rounds
@@ -991,12 +1174,19 @@ ibk_status step_chebyshev(ibk_diffusion_s& d, double gamma, const double* u, con
 	cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(double) * (kScalars + 1), s);
 	if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
 	launch_rhs(d, gamma, u, rhs, f, r[0], s);
+	const bool flat = d.ops.dims == 2;
 	const auto polynomial = [&](const double* rin, double* rout, int first) {
-		if (d.poly_wide)
-			polynomial_kernel<PolyWide><<<d.poly_grid, PolyWide::THREADS, PolyWide::BYTES, s>>>(
+		if (flat && d.poly_wide)
+			polynomial_plane_kernel<PlaneWide><<<d.poly_grid, PlaneWide::THREADS, 0, s>>>(d.ops, sc, rin, q, rout, z,
+			                                                                             d.partial, done, first, cw);
+		else if (flat)
+			polynomial_plane_kernel<PlaneSmall><<<d.poly_grid, PlaneSmall::THREADS, 0, s>>>(d.ops, sc, rin, q, rout, z,
+			                                                                               d.partial, done, first, cw);
+		else if (d.poly_wide)
+			polynomial_kernel<PolyWide><<<d.poly_grid, PolyWide::THREADS, poly_bytes<PolyWide>(), s>>>(
 				d.ops, sc, rin, q, rout, z, d.partial, done, d.poly_run, first, cw);
 		else
-			polynomial_kernel<PolySmall><<<d.poly_grid, PolySmall::THREADS, PolySmall::BYTES, s>>>(
+			polynomial_kernel<PolySmall><<<d.poly_grid, PolySmall::THREADS, poly_bytes<PolySmall>(), s>>>(
 				d.ops, sc, rin, q, rout, z, d.partial, done, d.poly_run, first, cw);
 	};
 	polynomial(r[0], r[1], 1);
@@ -1005,9 +1195,14 @@ ibk_status step_chebyshev(ibk_diffusion_s& d, double gamma, const double* u, con
 	const double* seen = nullptr;          // the test that stopped the loop
 	for (long long it = 0; !seen; ++it) {
 		const int a = (int) (it & 1), slot = (int) (it % (kLookAhead + 1));
-		direction_apply_kernel<<<d.dir_grid, kDirThreads, 0, s>>>(d.ops, sc, z, dv[a], dv[a ^ 1], x, q, d.partial, done,
-		                                                          d.dir_run, it == 0, d.tolerance, d.max_iterations,
-		                                                          d.host_tests + 2 * slot);
+		if (flat)
+			direction_plane_kernel<<<d.dir_grid, kDirThreads, 0, s>>>(d.ops, sc, z, dv[a], dv[a ^ 1], x, q, d.partial, done,
+			                                                          it == 0, d.tolerance, d.max_iterations,
+			                                                          d.host_tests + 2 * slot);
+		else
+			direction_apply_kernel<<<d.dir_grid, kDirThreads, 0, s>>>(d.ops, sc, z, dv[a], dv[a ^ 1], x, q, d.partial, done,
+			                                                          d.dir_run, it == 0, d.tolerance, d.max_iterations,
+			                                                          d.host_tests + 2 * slot);
 		if ((e = cudaEventRecord(d.tested[slot], s)) != cudaSuccess) return cuda_fail(e, "diffusion residual read");
 		polynomial(r[a ^ 1], r[a], 0);
 		if ((st = check_launch("diffusion iteration kernels")) != IBK_OK) return st;
@@ -1156,11 +1351,14 @@ ibk_status ibk_diffusion_create(ibk_plan plan, int component, const double robin
 	d->dir_grid = dim3(tiles(P0, kDirX), tiles(P1, kDirY), 1);
 	d->dir_run = pick_run((long long) d->dir_grid.x * d->dir_grid.y, P2, 1, (long long) kDirBlocks * p->num_sms).planes;
 	d->dir_grid.z = tiles(P2, d->dir_run);
-	// the wide tile's step takes kWideStep times as long as the small one's
+	// The wide tile's step takes kWideStep times as long as the small one's.  In two
+	// dimensions a step is short and the small tile's extra halo counts once its
+	// blocks no longer run all at once (see PlaneSmall).
+	const bool flat = g.dims == 2;
 	const dim3 wide(tiles(P0, PolyWide::X), tiles(P1, PolyWide::Y), 1), small(tiles(P0, PolySmall::X), tiles(P1, PolySmall::Y), 1);
 	const Run rw = pick_run((long long) wide.x * wide.y, P2, PolyWide::HALO, (long long) PolyWide::BLOCKS * p->num_sms);
 	const Run rs = pick_run((long long) small.x * small.y, P2, PolySmall::HALO, (long long) PolySmall::BLOCKS * p->num_sms);
-	d->poly_wide = kWideStep * rw.cost <= rs.cost;
+	d->poly_wide = flat ? (long long) small.x * small.y > 2LL * p->num_sms : kWideStep * rw.cost <= rs.cost;
 	d->poly_grid = d->poly_wide ? wide : small;
 	d->poly_run = (d->poly_wide ? rw : rs).planes;
 	d->poly_grid.z = tiles(P2, d->poly_run);
@@ -1182,9 +1380,9 @@ ibk_status ibk_diffusion_create(ibk_plan plan, int component, const double robin
 	for (cudaEvent_t& ev : d->tested)
 		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
 	if (e == cudaSuccess)
-		e = cudaFuncSetAttribute(polynomial_kernel<PolyWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, PolyWide::BYTES);
+		e = cudaFuncSetAttribute(polynomial_kernel<PolyWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, poly_bytes<PolyWide>());
 	if (e == cudaSuccess)
-		e = cudaFuncSetAttribute(polynomial_kernel<PolySmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, PolySmall::BYTES);
+		e = cudaFuncSetAttribute(polynomial_kernel<PolySmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, poly_bytes<PolySmall>());
 	if (e == cudaSuccess) e = cudaMemcpy(d->coef, host.data(), sizeof(double) * (size_t) total, cudaMemcpyHostToDevice);
 	if (e != cudaSuccess) {
 		cudaGetLastError();
