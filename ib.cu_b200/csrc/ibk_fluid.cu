@@ -608,9 +608,9 @@ __device__ __forceinline__ void advance(double delta, double* sc, int first)
 	}
 }
 
-// Time of one step of polynomial_kernel's wide tile over the small tile's, from
-// the solves timed above; it puts the line a little below 128^3 faces.
-constexpr double kWideStep = 1.5;
+// Time of one step of polynomial_kernel's wide tile over the small tile's (see
+// PolyWide).
+constexpr double kWideStep = 1.75;
 
 // Longest run of planes per block (bounds the tables along z).
 constexpr int kMaxRun = 64;
@@ -832,10 +832,12 @@ struct PolyTile {
 	static_assert(THREADS % 32 == 0, "whole warps");
 };
 // Of the wide tile's columns 74 % are the block's own, of the small tile's
-// half; the small one has four times the blocks.  With three rows a thread in
-// the wide tile (743 us): 512 x 256 x 512 faces 20.2 ms a solve against 23.4
-// ms, 256 x 128 x 256 3.43 against 3.57, 128^3 1.11 against 1.09, 117 x 234 x
-// 117 1.85 against 1.76, 64^3 0.49 against 0.46.
+// half; the small one has four times the blocks.  Milliseconds a solve, wide /
+// small: 512 x 256 x 512 faces 18.3 / 22.7, 256 x 128 x 256 2.86 / 3.26, 160^3 1.60
+// / 1.92, 128^3 1.06 / 1.04, 112^3 0.77 / 0.87, 104^3 0.69 / 0.72, 96^3 0.66 / 0.63,
+// 64^3 0.47 / 0.41, 8 x 512 x 512 3.05 / 2.49.  The cost that pick_run gives is
+// 1.53 times the wide tile's for the small one at 96^3, 1.71 at 128^3, 1.80 at
+// 104^3: the line lies between the last two.
 using PolyWide = PolyTile<64, 8, 4, 1>;
 using PolySmall = PolyTile<32, 16, 1, 2>;
 template <typename T> constexpr int poly_bytes() { return 6 * T::PLANE * (int) sizeof(double); }
