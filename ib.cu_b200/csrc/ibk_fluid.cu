@@ -608,7 +608,7 @@ __device__ __forceinline__ void advance(double delta, double* sc, int first)
 	}
 }
 
-// Time of one step of polynomial_kernel's wide tile over the small tile's (see
+// Time of one step of polynomial_kernel's wide tile over the others' (see
 // PolyWide).
 constexpr double kWideStep = 1.75;
 
@@ -831,15 +831,19 @@ struct PolyTile {
 	static constexpr int PLANE = EX * EY;
 	static_assert(THREADS % 32 == 0, "whole warps");
 };
-// Of the wide tile's columns 74 % are the block's own, of the small tile's
-// half; the small one has four times the blocks.  Milliseconds a solve, wide /
-// small: 512 x 256 x 512 faces 18.3 / 22.7, 256 x 128 x 256 2.86 / 3.26, 160^3 1.60
-// / 1.92, 128^3 1.06 / 1.04, 112^3 0.77 / 0.87, 104^3 0.69 / 0.72, 96^3 0.66 / 0.63,
+// Of the wide tile's columns 74 % are the block's own, of the small and the
+// tall tile's half; these have four times the blocks.  Milliseconds a solve,
+// wide / small: 512 x 256 x 512 faces 18.3 / 22.7, 256 x 128 x 256 2.86 / 3.26, 160^3
+// 1.60 / 1.92, 128^3 1.06 / 1.04, 112^3 0.77 / 0.87, 104^3 0.69 / 0.72, 96^3 0.66 / 0.63,
 // 64^3 0.47 / 0.41, 8 x 512 x 512 3.05 / 2.49.  The cost that pick_run gives is
 // 1.53 times the wide tile's for the small one at 96^3, 1.71 at 128^3, 1.80 at
-// 104^3: the line lies between the last two.
+// 104^3: the line lies between the last two.  The tall tile is for grids of a
+// few faces along x, most of which the small one spends on columns past the
+// end.
 using PolyWide = PolyTile<64, 8, 4, 1>;
 using PolySmall = PolyTile<32, 16, 1, 2>;
+using PolyTall = PolyTile<16, 32, 1, 2>;
+enum PolyKind { kPolyWide, kPolySmall, kPolyTall };
 template <typename T> constexpr int poly_bytes() { return 6 * T::PLANE * (int) sizeof(double); }
 
 struct ChebWeights { double w[4]; };
@@ -1143,7 +1147,7 @@ struct ibk_diffusion_s {
 	March march;                   // march_apply_kernel's grid
 	dim3 dir_grid, poly_grid;      // grids and planes per block of the Chebyshev loop's kernels
 	int dir_run = 1, poly_run = 1;
-	bool poly_wide = true;
+	PolyKind poly_kind = kPolyWide;
 	double* scalars = nullptr;     // device scalars of the loop, then the kernels' counter of finished blocks
 	double* host_tests = nullptr;                   // pinned: stop and iterations of each look-ahead slot
 	cudaEvent_t tested[kLookAhead + 1] = {};        // the kernel that writes each slot
@@ -1177,19 +1181,21 @@ ibk_status step_chebyshev(ibk_diffusion_s& d, double gamma, const double* u, con
 	if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
 	launch_rhs(d, gamma, u, rhs, f, r[0], s);
 	const bool flat = d.ops.dims == 2;
+	const auto march = [&](auto tile, const double* rin, double* rout, int first) {
+		using T = decltype(tile);
+		polynomial_kernel<T><<<d.poly_grid, T::THREADS, poly_bytes<T>(), s>>>(d.ops, sc, rin, q, rout, z, d.partial, done,
+		                                                                     d.poly_run, first, cw);
+	};
+	const auto plane = [&](auto tile, const double* rin, double* rout, int first) {
+		using T = decltype(tile);
+		polynomial_plane_kernel<T><<<d.poly_grid, T::THREADS, 0, s>>>(d.ops, sc, rin, q, rout, z, d.partial, done, first, cw);
+	};
 	const auto polynomial = [&](const double* rin, double* rout, int first) {
-		if (flat && d.poly_wide)
-			polynomial_plane_kernel<PlaneWide><<<d.poly_grid, PlaneWide::THREADS, 0, s>>>(d.ops, sc, rin, q, rout, z,
-			                                                                             d.partial, done, first, cw);
-		else if (flat)
-			polynomial_plane_kernel<PlaneSmall><<<d.poly_grid, PlaneSmall::THREADS, 0, s>>>(d.ops, sc, rin, q, rout, z,
-			                                                                               d.partial, done, first, cw);
-		else if (d.poly_wide)
-			polynomial_kernel<PolyWide><<<d.poly_grid, PolyWide::THREADS, poly_bytes<PolyWide>(), s>>>(
-				d.ops, sc, rin, q, rout, z, d.partial, done, d.poly_run, first, cw);
-		else
-			polynomial_kernel<PolySmall><<<d.poly_grid, PolySmall::THREADS, poly_bytes<PolySmall>(), s>>>(
-				d.ops, sc, rin, q, rout, z, d.partial, done, d.poly_run, first, cw);
+		switch (d.poly_kind) {
+		case kPolyWide: return flat ? plane(PlaneWide(), rin, rout, first) : march(PolyWide(), rin, rout, first);
+		case kPolySmall: return flat ? plane(PlaneSmall(), rin, rout, first) : march(PolySmall(), rin, rout, first);
+		case kPolyTall: return march(PolyTall(), rin, rout, first);
+		}
 	};
 	polynomial(r[0], r[1], 1);
 	ibk_status st = check_launch("diffusion set-up kernels");
@@ -1353,16 +1359,26 @@ ibk_status ibk_diffusion_create(ibk_plan plan, int component, const double robin
 	d->dir_grid = dim3(tiles(P0, kDirX), tiles(P1, kDirY), 1);
 	d->dir_run = pick_run((long long) d->dir_grid.x * d->dir_grid.y, P2, 1, (long long) kDirBlocks * p->num_sms).planes;
 	d->dir_grid.z = tiles(P2, d->dir_run);
-	// The wide tile's step takes kWideStep times as long as the small one's.  In two
-	// dimensions a step is short and the small tile's extra halo counts once its
-	// blocks no longer run all at once (see PlaneSmall).
+	// The tile of the cheapest run; the wide one's step takes kWideStep times as
+	// long as the others'.  In two dimensions a step is short and the small
+	// tile's extra halo counts once its blocks no longer run all at once (see
+	// PlaneSmall).
 	const bool flat = g.dims == 2;
-	const dim3 wide(tiles(P0, PolyWide::X), tiles(P1, PolyWide::Y), 1), small(tiles(P0, PolySmall::X), tiles(P1, PolySmall::Y), 1);
-	const Run rw = pick_run((long long) wide.x * wide.y, P2, PolyWide::HALO, (long long) PolyWide::BLOCKS * p->num_sms);
-	const Run rs = pick_run((long long) small.x * small.y, P2, PolySmall::HALO, (long long) PolySmall::BLOCKS * p->num_sms);
-	d->poly_wide = flat ? (long long) small.x * small.y > 2LL * p->num_sms : kWideStep * rw.cost <= rs.cost;
-	d->poly_grid = d->poly_wide ? wide : small;
-	d->poly_run = (d->poly_wide ? rw : rs).planes;
+	double best = -1.0;
+	const auto consider = [&](auto tile, PolyKind kind, double step) {
+		using T = decltype(tile);
+		const dim3 grid(tiles(P0, T::X), tiles(P1, T::Y), 1);
+		const Run run = pick_run((long long) grid.x * grid.y, P2, T::HALO, (long long) T::BLOCKS * p->num_sms);
+		if (best >= 0.0 && step * (double) run.cost >= best) return;
+		best = step * (double) run.cost;
+		d->poly_kind = kind;
+		d->poly_grid = grid;
+		d->poly_run = run.planes;
+	};
+	const bool rounds = (long long) tiles(P0, PolySmall::X) * tiles(P1, PolySmall::Y) > 2LL * p->num_sms;
+	if (!flat || rounds) consider(PolyWide(), kPolyWide, kWideStep);
+	if (!flat || !rounds) consider(PolySmall(), kPolySmall, 1.0);
+	if (!flat) consider(PolyTall(), kPolyTall, 1.0);
 	d->poly_grid.z = tiles(P2, d->poly_run);
 	for (const dim3& g : {d->march.grid, d->dir_grid, d->poly_grid})
 		if (g.y > 65535u || g.z > 65535u || size >= (1LL << 31)) {
@@ -1385,6 +1401,8 @@ ibk_status ibk_diffusion_create(ibk_plan plan, int component, const double robin
 		e = cudaFuncSetAttribute(polynomial_kernel<PolyWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, poly_bytes<PolyWide>());
 	if (e == cudaSuccess)
 		e = cudaFuncSetAttribute(polynomial_kernel<PolySmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, poly_bytes<PolySmall>());
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(polynomial_kernel<PolyTall>, cudaFuncAttributeMaxDynamicSharedMemorySize, poly_bytes<PolyTall>());
 	if (e == cudaSuccess) e = cudaMemcpy(d->coef, host.data(), sizeof(double) * (size_t) total, cudaMemcpyHostToDevice);
 	if (e != cudaSuccess) {
 		cudaGetLastError();

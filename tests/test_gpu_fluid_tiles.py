@@ -18,6 +18,8 @@ CASES = [((3, 6, 12), (0, 0, 0), 0), ((3, 6, 12), (0, 1, 0), 1), ((4, 8, 4), (1,
          ((26, 13, 52), (0, 1, 0), 0), ((27, 27, 27), (1, 0, 1), 1), ((59, 59, 118), (0, 1, 0), 0),
          ((59, 118), (0, 1), 0), ((174, 87, 87), (0, 0, 0), 2), ((174, 87, 87), (0, 1, 0), 1),
          ((174, 87, 87), (1, 1, 1), 0),
+         # few faces along x: tiles of 10 x 26
+         ((4, 400, 40), (1, 0, 1), 0), ((8, 400, 40), (0, 1, 0), 1),
          # two dimensions: tiles of 26 x 10 faces, more than 2 per SM of those: of 58 x 26
          ((3, 3), (0, 0), 0), ((4, 8), (1, 1), 0), ((26, 52), (0, 0), 1), ((27, 54), (1, 0), 1), ((348, 232), (0, 0), 0),
          ((348, 232), (1, 1), 1), ((464, 232), (0, 1), 0)]
