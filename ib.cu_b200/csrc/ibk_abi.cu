@@ -302,6 +302,7 @@ ibk_status ibk_plan_create(const ibk_domain* domain, int tag, int refinement, ib
 	cudaError_t e = cudaMalloc(&plan->d_status, sizeof(int) * 4);
 	if (e != cudaSuccess) { cudaGetLastError(); delete plan; return set_error(IBK_ERR_OUT_OF_MEMORY, "cudaMalloc failed"); }
 	cudaMemset(plan->d_status, 0, sizeof(int) * 4);
+	cudaStreamSynchronize(cudaStreamLegacy);     // the plan's calls may come on streams that do not wait for that one
 	*out = reinterpret_cast<ibk_plan>(plan);
 	return IBK_OK;
 }
@@ -469,6 +470,7 @@ ibk_status ibk_plan_check(ibk_plan handle)
 	if (e != cudaSuccess) return set_error(IBK_ERR_CUDA, std::string("cudaMemcpy: ") + cudaGetErrorString(e));
 	if (st[0] == 0) return IBK_OK;
 	cudaMemset(plan->d_status, 0, sizeof(st));
+	cudaStreamSynchronize(cudaStreamLegacy);
 	return set_error(IBK_ERR_DEVICE_CHECK, st[0] == 1 ? "a bounded device wait timed out" :
 	                 "a TMA precondition failed on the device (staged by plain loads instead)");
 }

@@ -1075,6 +1075,7 @@ ibk_status ibk_batch_check(ibk_batch handle)
 	if (s != IBK_OK) return s;
 	if (st[0] == 0) return IBK_OK;
 	cudaMemset(b->d_status, 0, sizeof(int) * 4);
+	cudaStreamSynchronize(cudaStreamLegacy);
 	return set_error(IBK_ERR_DEVICE_CHECK, "device check tripped (code " + std::to_string(st[0]) + ")");
 }
 

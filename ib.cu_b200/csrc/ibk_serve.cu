@@ -327,6 +327,8 @@ ibk_status ibk_server_admit(ibk_server handle, int member, int n, const double* 
 	if (st == IBK_OK && n > 0) st = cuda_ok(cudaMemcpy(m.xref, x, xb, cudaMemcpyHostToDevice), "cudaMemcpy");
 	if (st == IBK_OK) st = cuda_ok(cudaMemset(m.fs, 0, pbytes), "cudaMemset");
 	if (st == IBK_OK) st = cuda_ok(cudaMemset(m.x[1], 0, pbytes), "cudaMemset");
+	// the slots' streams do not wait for the default stream, which may be busy
+	if (st == IBK_OK) st = cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "cudaStreamSynchronize");
 	if (st != IBK_OK) { free_member(m); return st; }
 	m.admitted = true;
 	m.n = n;
@@ -467,6 +469,7 @@ ibk_status ibk_server_admit_from(ibk_server handle, int member, const char* path
 	for (int c = 0; c < s->dims && st == IBK_OK; ++c)
 		st = cuda_ok(cudaMemcpy(m.fe[c], grids[s->dims + c].data(), sizeof(double) * grids[s->dims + c].size(),
 		                        cudaMemcpyHostToDevice), "cudaMemcpy");
+	if (st == IBK_OK) st = cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), "cudaStreamSynchronize");
 	if (st != IBK_OK) {
 		// a member restored only in part is not left admitted: release it as
 		// retire does (nothing of it is in flight yet) and report the error

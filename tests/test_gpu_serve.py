@@ -160,3 +160,24 @@ def test_checkpoint_restores_a_member(ibk, cuda, tmp_path):
     assert np.array_equal(xa, xb)
     for u, v in zip(fa, fb):
         assert np.array_equal(u, v)
+
+
+def test_members_admitted_while_the_default_stream_is_busy(ibk, cuda):
+    """The slots' streams do not wait for the default stream: what admission
+    clears and copies there must be done before a step may start."""
+    import torch
+    ws = _members()[:3]
+    plans, ues = zip(*[_velocities(ibk, w, 400 + i) for i, w in enumerate(ws)])
+    quiet = _server(ibk, ws, ues, slots=2)
+    a = torch.ones(1 << 28, dtype=torch.float64, device=cuda)
+    for _ in range(40):                 # about 25 ms of copies
+        a.mul_(1.0)
+    busy = _server(ibk, ws, ues, slots=2)
+    for srv in (busy, quiet):
+        for i in range(len(ws)):
+            srv.submit(i)
+        srv.drain()
+    for i, w in enumerate(ws):
+        xa, fa = busy.read(i, w.n, plans[i].sizes())
+        xb, fb = quiet.read(i, w.n, plans[i].sizes())
+        assert np.array_equal(xa, xb) and all(np.array_equal(p, q) for p, q in zip(fa, fb))
