@@ -486,7 +486,11 @@ __device__ __forceinline__ bool grid_sums(double* v, double* part, unsigned* don
 	return true;
 }
 
-// Plane p on the z axis, at most three planes past its ends: wrapped on a
+// Points an axis has at least: the tiles' halos then reach no further than one
+// period past an end.
+constexpr int kMinPoints = 3;
+
+// Plane p on the z axis, at most kMinPoints planes past its ends: wrapped on a
 // periodic axis, -1 outside a wall.
 __device__ __forceinline__ int fold_plane(const AxisOps& a, int p)
 {
@@ -830,6 +834,7 @@ struct PolyTile {
 	static constexpr int EY = TY * ROWS, X = EX - 2 * HALO, Y = EY - 2 * HALO, THREADS = EX * TY;
 	static constexpr int PLANE = EX * EY;
 	static_assert(THREADS % 32 == 0, "whole warps");
+	static_assert(HALO <= kMinPoints, "fold_plane adds or subtracts one period");
 };
 // Of the wide tile's columns 74 % are the block's own, of the small and the
 // tall tile's half; these have four times the blocks.  Milliseconds a solve,
@@ -1315,7 +1320,7 @@ ibk_status ibk_diffusion_create(ibk_plan plan, int component, const double robin
 	int off = 0;
 	for (int a = 0; a < g.dims; ++a) {
 		const int P = cg.points[a];
-		if (P < 3) {
+		if (P < kMinPoints) {
 			delete d;
 			return set_error(IBK_ERR_INVALID_ARGUMENT, "each axis needs at least 3 points");
 		}
