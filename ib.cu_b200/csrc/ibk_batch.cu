@@ -226,7 +226,7 @@ batch_spread_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __re
 
 // Persistent FP64 spread over the active instances' (tile, component) items.
 template <typename D, int DIMS, bool OWNERS = s64_owners<D, DIMS>()>
-__global__ void __launch_bounds__(s64_threads<OWNERS>(), s64_ctas<OWNERS>())
+__global__ void __launch_bounds__(s64_threads<OWNERS>(), s64_ctas<D, OWNERS>())
 batch_spread64_kernel(const BatchInst* __restrict__ insts, BatchTable t, int* __restrict__ next,
                       const PointRec* __restrict__ recs, const int* __restrict__ off, int step)
 {

@@ -20,7 +20,8 @@
 // polynomial in H = I~ - lambda L on its Gershgorin interval
 // (include/solvers/chebpcg.h, include/solvers/preconditioners/chebyshev.h,
 // include/algo/chebyshev.h, include/algo/gershgorin.h), or, selectable, a
-// Jacobi preconditioner.  FP64, compiled without contraction.
+// Jacobi preconditioner.  FP64, compiled without contraction; the kernels of
+// the Chebyshev loop use fused multiply-adds, each written out.
 #include <algorithm>
 #include <cmath>
 #include <string>

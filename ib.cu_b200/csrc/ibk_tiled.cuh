@@ -6,8 +6,10 @@
 // spread_tile  -- owner computes.  The CTA visits every point whose stencil
 //   can touch its tile (its own bins plus the neighbours' bins whose reach
 //   class points at it), accumulates the in-tile contributions in shared
-//   memory, and writes every face of its tile exactly once (zeros included).
-//   No global atomics, no zero-fill pass: each face is written by one CTA.
+//   memory, and writes every face of its tile exactly once (zeros included):
+//   no global atomics, no zero-fill pass.  The exception is an FP64 spread whose
+//   few, full tiles are split over several CTAs: these add their sums to faces
+//   zeroed before.
 //     FP32C: one CTA per tile for every component.  FP32 weights and
 //            products, each rounded once to a per-(tile, component) fixed
 //            point and summed exactly with 32-bit integer shared atomics
@@ -863,6 +865,11 @@ __device__ __forceinline__ void add_candidates64(const GridGeom& g, const TileGe
 	for (int it = threadIdx.x; it < ncand; it += NT) {
 		const PointRec rec = load_rec(recs + range_walk(rt, r, it));
 		const int sft = rt.shift[r], p = rec.p - pbase;
+		// loads first: the masks are formed while they are in flight
+		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
+		double z[DIMS];
+#pragma unroll
+		for (int d = 0; d < DIMS; ++d) z[d] = __ldg(x + (size_t) d * n + p);
 		int l[DIMS];
 		unsigned mk[DIMS];
 		bool any = true;
@@ -873,11 +880,9 @@ __device__ __forceinline__ void add_candidates64(const GridGeom& g, const TileGe
 			any = any && mk[d] != 0u;
 		}
 		if (!any) continue;
-		const double f = __dmul_rn(g.res, __ldg(fl + (size_t) c * n + p));
 		double w[DIMS][M];
 #pragma unroll
-		for (int d = 0; d < DIMS; ++d)
-			tile_weights64<D>(axis_step<M>(g, cg, d, __ldg(x + (size_t) d * n + p)).delta, mk[d], w[d]);
+		for (int d = 0; d < DIMS; ++d) tile_weights64<D>(axis_step<M>(g, cg, d, z[d]).delta, mk[d], w[d]);
 #pragma unroll
 		for (int m0 = 0; m0 < M; ++m0) w[0][m0] = __dmul_rn(w[0][m0], f);
 		if (!wrap_any) {
@@ -1144,8 +1149,8 @@ __device__ __forceinline__ void spread_tile64(const GridGeom& g, const TileGeom&
 // takes it: the owners' lanes are 64 nodes in two rounds, and two warps cannot
 // prepare dearer weights in time.  128 x 64 x 128 cells, 124,700 points, in us,
 // binning included, a general form of the owners / this one: bspline<1> 104 /
-// 59, bspline<2> 134 / 99, bspline<4> 1589 / 541, bspline<5> 7162 / 2107, peskin
-// 223 / 180, roma 214 / 111, cosine 272 / 195, hat 102 / 58.  In two dimensions
+// 57, bspline<2> 134 / 99, bspline<4> 1589 / 538, bspline<5> 7162 / 2112, peskin
+// 223 / 178, roma 214 / 108, cosine 272 / 193, hat 102 / 55.  In two dimensions
 // a stencil has at most 36 nodes and a tile few faces, so the owners would
 // work through a long chain with half of their lanes idle (24 outlines of 160
 // points on 240 x 120 cells: 20 us against 30).
@@ -1185,7 +1190,7 @@ __device__ __forceinline__ void spread_tile64_atomic(const GridGeom& g, const Ti
 constexpr bool spread64_owners(int kind, int order, int dims) { return kind == kBspline && order == 3 && dims == 3; }
 template <typename D, int DIMS> constexpr bool s64_owners() { return DIMS == 3 && std::is_same_v<D, Delta<kBspline, 3>>; }
 template <bool OWNERS> constexpr int s64_threads() { return OWNERS ? kS64Threads : kTileThreads; }
-template <bool OWNERS> constexpr int s64_ctas() { return OWNERS ? 4 : 3; }
+template <typename D, bool OWNERS> constexpr int s64_ctas() { return OWNERS || D::M == 2 ? 4 : 3; }
 
 template <typename D, int DIMS, bool OWNERS>
 __device__ __forceinline__ void spread_any64(const GridGeom& g, const TileGeom& tg, int n, const double* __restrict__ x,
@@ -1227,9 +1232,11 @@ spread_tile_kernel(GridGeom g, TileGeom tg, const PointRec* __restrict__ recs, c
 }
 
 // grid: (tile, component, part); of the owners' form four CTAs of 52 KB per SM
-// at 16^3 tiles, of the other three (85 registers).
+// at 16^3 tiles, of the other three (80 registers), four for stencils of two
+// points, which need 65 (one red cell on 160^3, mostly empty tiles: hat 62 us with
+// three).
 template <typename D, int DIMS, bool OWNERS>
-__global__ void __launch_bounds__(s64_threads<OWNERS>(), s64_ctas<OWNERS>())
+__global__ void __launch_bounds__(s64_threads<OWNERS>(), s64_ctas<D, OWNERS>())
 spread_tile64_kernel(GridGeom g, TileGeom tg, int n, const double* __restrict__ x, const double* __restrict__ fl,
                      const PointRec* __restrict__ recs, const int* __restrict__ off, CompPtrs fe)
 {
